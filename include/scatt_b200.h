@@ -89,6 +89,17 @@ int scatt_inverse_batched(int n, int count, const double* A, double* out,
 int scatt_inverse_batched_noalloc(int n, int count, const double* A, double* out,
                                   int symmetrize, int* status);
 
+/* Batched inverse of `count` symmetric n x n matrices (contiguous, ld = n,
+ * both triangles given; orders up to 8192), exactly symmetric, by the
+ * blocked symmetric sweep that the solver runs on S(n) and R(n) under the
+ * automatic scheme: n^3 flops each, half of scatt_inverse_batched's.
+ * status as for scatt_inverse_batched; mode (may be NULL) receives per
+ * matrix how it was finished: 0 the sweep alone, 1 or 2 with that many Newton
+ * steps after it (its intermediate inverses had grown), 3 a pivoted
+ * elimination.  Replaces inverse_symmetric_indefinite
+ * (src/scatt/LapackInverse.hpp:120-178). */
+int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* out, int* status, int* mode);
+
 /* C = alpha op(A) op(B) + beta C on the device, host buffers (op: 0 = N, 1 = T). */
 int scatt_dgemm(int opA, int opB, int M, int N, int K, double alpha,
                 const double* A, int lda, const double* B, int ldb,

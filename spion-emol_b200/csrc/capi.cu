@@ -7,6 +7,7 @@
 
 #include "angular.hpp"
 #include "common.cuh"
+#include "sym_rescue.cuh"
 #include "devbuf.cuh"
 #include "riccati.cuh"
 
@@ -197,6 +198,64 @@ int scatt_inverse_batched(int n, int count, const double* A, double* out, int sy
             return SCATT_ERR_NONFINITE;
         }
     }
+    return SCATT_OK;
+}
+
+int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* out, int* status, int* mode) {
+    if (n <= 0 || count <= 0 || !A || !out) {
+        set_last_error("scatt_inverse_symmetric_batched: bad arguments");
+        return SCATT_ERR_ARG;
+    }
+    if (n > 8192 || count > 65535) {
+        set_last_error("scatt_inverse_symmetric_batched: order above 8192 or more than 65535 matrices");
+        return SCATT_ERR_SIZE;
+    }
+    SCATT_TRY(require_device());
+    const size_t nn = (size_t)n * n, al = 31;
+    const size_t ws = (sym_work_doubles(n) + al) & ~al, ps = sym_panel_doubles(n);
+    DevBuf<double> dA, dW, dO, dP;
+    DevBuf<int> dst;
+    DevBuf<unsigned long long> dmag;
+    DevBuf<unsigned> dbar;
+    SCATT_TRY(dA.alloc(nn * count));
+    SCATT_TRY(dW.alloc(ws * count));
+    SCATT_TRY(dO.alloc(nn * count));
+    SCATT_TRY(dP.alloc(ps * count));
+    SCATT_TRY(dst.alloc(2 * (size_t)count));
+    SCATT_TRY(dmag.alloc(4 * (size_t)count));
+    SCATT_TRY(dbar.alloc(1));
+    SCATT_TRY(dbar.zero());
+    SCATT_CUDA_TRY(cudaMemcpy(dA.p, A, nn * count * sizeof(double), cudaMemcpyHostToDevice));
+    SCATT_TRY(dmag.zero());
+    std::vector<SymEntry> ent(count);
+    const size_t T = sym_tiles_of(n);
+    for (int b = 0; b < count; ++b) {
+        double* P = dP.p + ps * b;
+        ent[b] = SymEntry{dA.p + nn * b, dW.p + ws * b, P, P + T * SYM_TILE, P + 2 * T * SYM_TILE,
+                          dO.p + nn * b, dmag.p + 4 * b, dst.p + 2 * b, n, n};
+    }
+    DevBuf<SymEntry> dent;
+    SCATT_TRY(dent.upload(ent));
+    SCATT_TRY(sym_pack_batched(dent.p, count, n, 0));
+    SCATT_TRY(sym_sweep_batched(dent.p, count, n, 0));
+    SCATT_TRY(sym_rescue_batched(dent.p, count, dbar.p, 0));
+    SCATT_CUDA_TRY(cudaDeviceSynchronize());
+    SCATT_CUDA_TRY(cudaMemcpy(out, dO.p, nn * count * sizeof(double), cudaMemcpyDeviceToHost));
+    std::vector<int> st(2 * count);
+    SCATT_CUDA_TRY(cudaMemcpy(st.data(), dst.p, st.size() * sizeof(int), cudaMemcpyDeviceToHost));
+    if (status) std::memcpy(status, st.data(), st.size() * sizeof(int));
+    if (mode) {
+        std::vector<unsigned long long> mg(4 * (size_t)count);
+        SCATT_CUDA_TRY(cudaMemcpy(mg.data(), dmag.p, mg.size() * sizeof(mg[0]), cudaMemcpyDeviceToHost));
+        for (int b = 0; b < count; ++b) mode[b] = (int)mg[4 * (size_t)b + 3];
+    }
+    for (int b = 0; b < count; ++b)
+        if (st[2 * b] != DEV_OK) {
+            set_last_error("scatt_inverse_symmetric_batched: " +
+                           std::string(st[2 * b] == DEV_SINGULAR ? "singular" : "non-finite") + " pivot in matrix " +
+                           std::to_string(b) + " at column " + std::to_string(st[2 * b + 1]));
+            return st[2 * b] == DEV_SINGULAR ? SCATT_ERR_SINGULAR : SCATT_ERR_NONFINITE;
+        }
     return SCATT_OK;
 }
 

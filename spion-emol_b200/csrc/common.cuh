@@ -50,6 +50,31 @@ inline int cuda_status(cudaError_t e, const char* what) {
 std::atomic<unsigned long long>& launch_counter();
 #define SCATT_COUNT_LAUNCH(n) (::scatt::launch_counter().fetch_add((n), std::memory_order_relaxed))
 
+// Launch that may be scheduled while the stream's previous kernel still runs
+// (programmatic dependent launch): the grid's set-up, 1 to 2 us of a chain of
+// short kernels, overlaps the previous kernel's end.  A kernel launched so
+// calls dep_sync() first in every thread, before any return: it waits for
+// the previous grid's completion and memory, then lets the next grid be
+// scheduled.  In a plainly launched kernel dep_sync() does nothing.
+template <class... P, class... A>
+cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void dep_sync() {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 // Device-side status codes written into per-matrix status words.
 enum DeviceStatus : int {
     DEV_OK = 0,

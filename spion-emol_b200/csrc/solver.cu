@@ -40,6 +40,7 @@
 #include "riccati.cuh"
 #include "scan.cuh"
 #include "step_kernels.cuh"
+#include "sym_rescue.cuh"
 #include "tables.hpp"
 
 namespace scatt {
@@ -112,6 +113,7 @@ __device__ __forceinline__ void build_V_pair(const BatchDev& b, int p, int n, do
 // V of every group's chunk: grid (pairs, groups, SCHUR_CHUNK), one thread per
 // channel pair (mu' <= mu).
 __global__ void k_build_V(BatchDev b) {
+    dep_sync();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const GroupDev& g = b.grp[blockIdx.y];
     const int j = blockIdx.z;
@@ -128,6 +130,7 @@ __global__ void k_build_V_at(BatchDev b, int n, double* V) {
 // diagonal of V(n + 1) for the groups whose step n = n0 + j is inside the
 // analytic start of the recurrence: grid (channels, groups).
 __global__ void k_vdiag(BatchDev b, int j) {
+    dep_sync();
     const int mu = blockIdx.x * blockDim.x + threadIdx.x;
     const GroupDev& g = b.grp[blockIdx.y];
     if (mu >= b.Np_max || g.n0 < 0 || j >= g.C || g.n0 + j >= b.n_start) return;
@@ -189,6 +192,7 @@ __device__ __forceinline__ void build_B_row(const BatchDev& b, int row, int n, d
 
 // B, Bs, D^-1 of every group's chunk: grid (rows, groups, SCHUR_CHUNK).
 __global__ void k_build_B(BatchDev b) {
+    dep_sync();
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     const GroupDev& g = b.grp[blockIdx.y];
     const int j = blockIdx.z;
@@ -226,47 +230,38 @@ __device__ __forceinline__ double* gacc_at(const BatchDev& b, const EnergyDev& d
     return (n & 1) ? d.G1 : d.G0;
 }
 
-// Entries of one chunk's Schur GEMM and inverse, index j * count + e.
-// Steps outside a slot's chunk get empty entries (M = 0, n = 0), which the
-// GEMM and inverse kernels skip; so do steps past n_transition for the GEMM.
-__global__ void k_prepare_schur(BatchDev b) {
+// Entry of a symmetric inverse of order n (ld n throughout), its magnitudes cleared.
+__device__ __forceinline__ SymEntry sym_entry(double* A, double* W, double* panel, double* out,
+                                              unsigned long long* mag, int* status, int n) {
+    const size_t T = sym_tiles_of(n);
+    mag[0] = mag[1] = mag[2] = mag[3] = 0;
+    return SymEntry{A, W, panel, panel + T * SYM_TILE, panel + 2 * T * SYM_TILE, out, mag, status, n, n};
+}
+
+// Fills a chunk's GEMM and inverse entries, index j * count + e (pointer
+// bookkeeping only; one launch for its SCHUR_CHUNK steps, which read nothing
+// that the chunk changes).  Entries of steps outside a slot's chunk, and of
+// stages a step does not take, are empty (M = 0, n = 0): the kernels skip them.
+__global__ void k_prepare(BatchDev b) {
+    dep_sync();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx <= SCHUR_CHUNK) b.barrier[idx] = 0;
     if (idx >= b.count * SCHUR_CHUNK) return;
     const int j = idx / b.count, e = idx % b.count;
     EnergyDev& d = b.ed[e];
     const int n = step_of(b, d, j);
-    const int Np = d.Np, Nf = b.Nf;
+    const int Np = d.Np, Nt = d.Nt, Nf = b.Nf, K = b.Krows;
     const size_t np2 = (size_t)Np * Np;
     double* S = d.S + j * np2;
     const GemmEntry none{nullptr, nullptr, nullptr, 0, 0, 0, 1, 1, 1, 0.0, 1.0};
+    GemmEntry *gmG1 = b.gmG + 2 * (size_t)j * b.count + e, *gmG2 = gmG1 + b.count;
     if (n < 0) {
-        b.gmS[idx] = none;
+        b.gmS[idx] = b.gmT[idx] = b.gmF[idx] = *gmG1 = *gmG2 = b.gmG3[idx] = b.gmGA[idx] = none;
         b.gjS[idx] = GjEntry{S, S, S, d.sigS, d.ridS, d.stS + 4 * j, 0, 1, 1, d.PS, d.sgS};
+        b.gjR[idx] = GjEntry{d.Ra, d.Rw, d.Ra, d.sigR, d.ridR, d.stR + 4 * j, 0, 1, 1, d.PR, d.sgR};
+        b.syS[idx].n = b.syR[idx].n = 0;
         return;
     }
-    const bool exch = n < b.n_tr && Nf > 0;
-    // Bs B^T = B D^-1 B^T and A are symmetric: lower tiles only, mirrored
-    b.gmS[idx] = exch ? GemmEntry{Bs_of(b, d, j), B_of(b, d, j), S, Np, Np, Nf, b.Np_max, b.Np_max, Np, -1.0, 1.0, 1}
-                      : none;
-    b.gjS[idx] = GjEntry{S, d.Sw + j * np2, sinv_at(b, d, n, j), d.sigS + (size_t)j * Np,
-                         d.ridS + (size_t)j * Np, d.stS + 4 * j, Np, Np, Np,
-                         d.PS + (size_t)j * 4 * GJ_WINDOW_MAX * Np, d.sgS + (size_t)j * 4 * Np};
-}
-
-// Fills the per-step GEMM / GJ entry arrays of chunk position j (pointer
-// bookkeeping only); entries a slot does not take this step are empty.
-__global__ void k_prepare(BatchDev b, int j) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= b.count) return;
-    EnergyDev& d = b.ed[e];
-    const int n = step_of(b, d, j);
-    const GemmEntry none{nullptr, nullptr, nullptr, 0, 0, 0, 1, 1, 1, 0.0, 1.0};
-    if (n < 0) {
-        b.gmT[e] = b.gmF[e] = b.gmG1[e] = b.gmG2[e] = b.gmG3[e] = b.gmGA[e] = none;
-        b.gjR[e] = GjEntry{d.Ra, d.Rw, d.Ra, d.sigR, d.ridR, d.stR, 0, 1, 1, d.PR, d.sgR};
-        return;
-    }
-    const int Np = d.Np, Nt = d.Nt, Nf = b.Nf, K = b.Krows;
     const bool exch = n < b.n_tr && Nf > 0;
     const bool sweep = n <= b.N - 1;
     double* sinv = sinv_at(b, d, n, j);
@@ -275,24 +270,33 @@ __global__ void k_prepare(BatchDev b, int j) {
     double* gnext = gacc_at(b, d, n + 1);
     const double* Bs = Bs_of(b, d, j);
     const double* Cn = (n < b.n_pts) ? b.Ctab + (size_t)n * K * b.Np_max : nullptr;
-    b.gmT[e] = exch ? GemmEntry{sinv, Bs, d.T, Np, Nf, Np, Np, b.Np_max, Np, 1.0, 0.0} : none;
+    // Bs B^T = B D^-1 B^T and A are symmetric: lower tiles only, mirrored
+    b.gmS[idx] = exch ? GemmEntry{Bs, B_of(b, d, j), S, Np, Np, Nf, b.Np_max, b.Np_max, Np, -1.0, 1.0, 1} : none;
+    b.gjS[idx] = GjEntry{S, d.Sw + j * b.sw_stride, sinv, d.sigS + (size_t)j * Np, d.ridS + (size_t)j * Np,
+                         d.stS + 4 * j, Np, Np, Np, d.PS + j * b.ps_stride, d.sgS + (size_t)j * 4 * Np};
+    b.syS[idx] = sym_entry(S, d.Sw + j * b.sw_stride, d.PS + j * b.ps_stride, sinv,
+                           b.mag + 4 * ((size_t)b.count * SCHUR_CHUNK + idx), d.stS + 4 * j, Np);
+    b.gmT[idx] = exch ? GemmEntry{sinv, Bs, d.T, Np, Nf, Np, Np, b.Np_max, Np, 1.0, 0.0} : none;
     // F = Bs^T Sinv Bs is symmetric: lower tiles only, mirrored
-    b.gmF[e] = exch ? GemmEntry{Bs, d.T, d.F, Nf, Nf, Np, b.Np_max, Np, Nf, 1.0, 0.0, 1} : none;
-    b.gmG1[e] = (sweep && Cn) ? GemmEntry{Cn, sinv, gcur, K, Np, Np, K, Np, K, 1.0, 1.0} : none;
-    b.gmG2[e] = (sweep && Cn && exch) ? GemmEntry{Cn, d.T, gcur + (size_t)Np * K, K, Nf, Np, K, Np, K, -1.0, 1.0}
-                                      : none;
-    b.gmG3[e] = sweep ? GemmEntry{gcur, rinv, gnext, K, Nt, Nt, K, Nt, K, 1.0, 0.0} : none;
+    b.gmF[idx] = exch ? GemmEntry{Bs, d.T, d.F, Nf, Nf, Np, b.Np_max, Np, Nf, 1.0, 0.0, 1} : none;
+    *gmG1 = (sweep && Cn) ? GemmEntry{Cn, sinv, gcur, K, Np, Np, K, Np, K, 1.0, 1.0} : none;
+    *gmG2 = (sweep && Cn && exch) ? GemmEntry{Cn, d.T, gcur + (size_t)Np * K, K, Nf, Np, K, Np, K, -1.0, 1.0} : none;
+    b.gmG3[idx] = sweep ? GemmEntry{gcur, rinv, gnext, K, Nt, Nt, K, Nt, K, 1.0, 0.0} : none;
     // the fit accumulation G_A(n)^T = H_A(n)^T Rinv(n) over n_s <= n <= N - 1
-    b.gmGA[e] = (d.GA0 && n >= b.n_s && sweep)
-                    ? GemmEntry{(n & 1) ? d.GA1 : d.GA0, rinv, (n & 1) ? d.GA0 : d.GA1, 2 * Np, Nt, Nt, 2 * Np, Nt,
-                                2 * Np, 1.0, 0.0}
-                    : none;
-    b.gjR[e] = GjEntry{d.Ra, d.Rw, rinv, d.sigR, d.ridR, d.stR, n >= b.n_start ? Nt : 0, Nt, Nt, d.PR, d.sgR};
+    b.gmGA[idx] = (d.GA0 && n >= b.n_s && sweep)
+                      ? GemmEntry{(n & 1) ? d.GA1 : d.GA0, rinv, (n & 1) ? d.GA0 : d.GA1, 2 * Np, Nt, Nt, 2 * Np, Nt,
+                                  2 * Np, 1.0, 0.0}
+                      : none;
+    const bool inv = n >= b.n_start;
+    b.gjR[idx] = GjEntry{d.Ra, d.Rw, rinv, d.sigR, d.ridR, d.stR + 4 * j, inv ? Nt : 0, Nt, Nt, d.PR, d.sgR};
+    if (inv) b.syR[idx] = sym_entry(d.Ra, d.Rw, d.PR, rinv, b.mag + 4 * (size_t)idx, d.stR + 4 * j, Nt);
+    else b.syR[idx].n = 0;
 }
 
 // A = (1 + h^2 E / 6) I - h^2/6 V(n) into Schur slot j (SchurInverter.cpp:253-261);
 // grid (x, slots, SCHUR_CHUNK).
 __global__ void k_init_S(BatchDev b) {
+    dep_sync();
     const int e = blockIdx.y, j = blockIdx.z;
     const EnergyDev& d = b.ed[e];
     if (step_of(b, d, j) < 0) return;
@@ -329,6 +333,7 @@ __device__ double block_min(double v, double* red) {
 // c I).  which = 0: A (also records delta_A), 1: S = A_shifted - Bs B^T
 // (exchange steps only).  Grid (slots, SCHUR_CHUNK); steps n >= stab_n skip.
 __global__ void k_stab(BatchDev b, int which) {
+    dep_sync();
     const int e = blockIdx.x, slot = blockIdx.y;
     EnergyDev& d = b.ed[e];
     const int n = step_of(b, d, slot);
@@ -365,39 +370,77 @@ __global__ void k_stab(BatchDev b, int which) {
         for (int i = threadIdx.x; i < Np; i += blockDim.x) S[i + (size_t)i * Np] += delta;
 }
 
-// R = 12 W^-1 - 10 I - Rinv_prev, W^-1 = [[Sinv, -T], [-T^T, D^-1 + F]];
-// slots whose step is inside the analytic start skip.
+// Element (i, jc) of R = 12 W^-1 - 10 I - Rinv_prev, W^-1 = [[Sinv, -T], [-T^T, D^-1 + F]].
+struct RElem {
+    const double *sinv, *T, *F, *Dinv, *prev;
+    int Np, Nt, Nf;
+    bool exch;
+    __device__ __forceinline__ RElem(const BatchDev& b, const EnergyDev& d, int n, int j)
+        : sinv(sinv_at(b, d, n, j)), T(d.T), F(d.F), Dinv(Dinv_of(b, d, j)), prev(rinv_at(b, d, n - 1)), Np(d.Np),
+          Nt(d.Nt), Nf(b.Nf), exch(n < b.n_tr) {}
+    __device__ __forceinline__ double operator()(int i, int jc) const {
+        double w;
+        if (i < Np && jc < Np) w = sinv[i + (size_t)jc * Np];
+        else if (i < Np) w = exch ? -T[i + (size_t)(jc - Np) * Np] : 0.0;
+        else if (jc < Np) w = exch ? -T[jc + (size_t)(i - Np) * Np] : 0.0;
+        else {
+            const int fi = i - Np, fj = jc - Np;
+            w = (fi == fj) ? Dinv[fi] : 0.0;
+            if (exch) w += F[fi + (size_t)fj * Nf];
+        }
+        const double u = 12.0 * w - ((i == jc) ? 10.0 : 0.0);
+        return u - prev[i + (size_t)jc * Nt];
+    }
+};
+
+// R(n) into Ra, column-major; slots whose step is inside the analytic start skip.
 __global__ void k_assemble_R(BatchDev b, int j) {
+    dep_sync();
     const int e = blockIdx.y;
     const EnergyDev& d = b.ed[e];
     const int n = step_of(b, d, j);
     if (n < b.n_start) return;                 // also n < 0
-    const int Np = d.Np, Nt = d.Nt, Nf = b.Nf;
-    const bool exch = n < b.n_tr;
-    const double* sinv = sinv_at(b, d, n, j);
-    const double* Dinv = Dinv_of(b, d, j);
-    const double* prev = rinv_at(b, d, n - 1);
+    const RElem R(b, d, n, j);
+    const int Nt = d.Nt;
     const long total = (long)Nt * Nt;
     for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
-         idx += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(idx % Nt), jc = (int)(idx / Nt);
-        double w;
-        if (i < Np && jc < Np) w = sinv[i + (size_t)jc * Np];
-        else if (i < Np) w = exch ? -d.T[i + (size_t)(jc - Np) * Np] : 0.0;
-        else if (jc < Np) w = exch ? -d.T[jc + (size_t)(i - Np) * Np] : 0.0;
-        else {
-            const int fi = i - Np, fj = jc - Np;
-            w = (fi == fj) ? Dinv[fi] : 0.0;
-            if (exch) w += d.F[fi + (size_t)fj * Nf];
-        }
-        const double u = 12.0 * w - ((i == jc) ? 10.0 : 0.0);
-        d.Ra[idx] = u - prev[idx];
+         idx += (long)gridDim.x * blockDim.x)
+        d.Ra[idx] = R((int)(idx % Nt), (int)(idx / Nt));
+}
+
+// The same for one entry of a rescue (sym_rescue_kernel).
+struct RSource {
+    BatchDev b;
+    int j;
+    __device__ __forceinline__ void operator()(int e, const SymEntry& s, int first, int stride) const {
+        const EnergyDev& d = b.ed[e];
+        const RElem R(b, d, step_of(b, d, j), j);
+        const long total = (long)s.n * s.n;
+        for (long idx = first; idx < total; idx += stride) s.A[idx] = R((int)(idx % s.n), (int)(idx / s.n));
     }
+};
+
+// R(n) packed for the symmetric sweep; grid (tiles, slots).  Bound by HBM:
+// it reads Sinv, T, F and Rinv(n - 1) once (the lower triangle's half of the
+// symmetric ones) and writes the triangle's tiles.
+__global__ void __launch_bounds__(SYM_THREADS) k_assemble_R_tiles(BatchDev b, int j) {
+    dep_sync();
+    extern __shared__ double smem[];
+    const int e = blockIdx.y;
+    const SymEntry s = b.syR[(size_t)j * b.count + e];
+    const int T = sym_tiles_of(s.n);
+    if ((int)blockIdx.x >= T * (T + 1) / 2) return;
+    const EnergyDev& d = b.ed[e];
+    const RElem R(b, d, step_of(b, d, j), j);
+    // the sources are symmetric: taken transposed, consecutive lanes read consecutive rows
+    sym_pack_tile(s, blockIdx.x, *reinterpret_cast<SymDiagShared*>(smem),
+                  [&R](int gi, int gj) { return R(gj, gi); });
 }
 
 // Analytic diagonal Rinv for 1 <= n < n_start, 0 at n = 0
 // (ForwardRPropagator.cpp:78-134): zero fill, then k_analytic_R_diag.
 __global__ void k_analytic_R(BatchDev b, int j) {
+    dep_sync();
     const int e = blockIdx.y;
     const EnergyDev& d = b.ed[e];
     const int n = step_of(b, d, j);
@@ -410,6 +453,7 @@ __global__ void k_analytic_R(BatchDev b, int j) {
 }
 
 __global__ void k_analytic_R_diag(BatchDev b, int j) {
+    dep_sync();
     const int e = blockIdx.y;
     const EnergyDev& d = b.ed[e];
     const int n = step_of(b, d, j);
@@ -448,18 +492,22 @@ __global__ void k_analytic_R_diag(BatchDev b, int j) {
     }
 }
 
-// sticky per-slot error: first failing inversion (step, code); which = 0:
-// the Schur inverse of chunk position j, 1: the R^-1 of position j.
-__global__ void k_collect(BatchDev b, int j, int which) {
+// sticky per-slot error: the chunk's first failing inversion (step, code),
+// Schur inverse before R^-1 at each step; runs at the end of the chunk.
+__global__ void k_collect(BatchDev b) {
+    dep_sync();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= b.count) return;
     EnergyDev& d = b.ed[e];
-    const int n = step_of(b, d, j);
-    if (n < 0 || (which == 1 && n < b.n_start)) return;
-    const int st = which ? d.stR[0] : d.stS[4 * j];
-    if (st != 0 && d.err_code == 0) {
-        d.err_code = (st == DEV_SINGULAR) ? SCATT_ERR_SINGULAR : SCATT_ERR_NONFINITE;
-        d.err_step = n;
+    for (int j = 0; j < SCHUR_CHUNK && d.err_code == 0; ++j) {
+        const int n = step_of(b, d, j);
+        if (n < 0) break;
+        int st = d.stS[4 * j];
+        if (st == 0 && n >= b.n_start) st = d.stR[4 * j];
+        if (st != 0) {
+            d.err_code = (st == DEV_SINGULAR) ? SCATT_ERR_SINGULAR : SCATT_ERR_NONFINITE;
+            d.err_step = n;
+        }
     }
 }
 
@@ -518,6 +566,7 @@ __global__ void k_ab_weights(BatchDev b, int e0) {
 
 // H_A(n)^T = G_A(n-1)^T + D_AB(n) [Sinv, -T] on the fit window; grid (x, slots)
 __global__ void k_acc_ab(BatchDev b, int j) {
+    dep_sync();
     const EnergyDev& d = b.ed[blockIdx.y];
     const int n = step_of(b, d, j);
     if (n < b.n_s || n > b.ne_fit || !d.GA0) return;
@@ -559,6 +608,7 @@ __global__ void k_ab_closed(const AbEntry* __restrict__ ents, const int* l_of_mu
 // End of a chunk: every running group moves on by its chunk's length; a
 // group whose chunk reached the stop step stops (n0 = -1).
 __global__ void k_advance(BatchDev b) {
+    dep_sync();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= b.ngroups) return;
     GroupDev& G = b.grp[g];
@@ -1367,6 +1417,10 @@ int ensure_stab(Context& ctx, const scatt_solve_opts& o, int l_cont, const doubl
     return SCATT_OK;
 }
 
+// Doubles of the panel buffers of one inverse of order n: the Gauss-Jordan
+// windows (four, with the look-ahead) or the symmetric sweep's P, M and D.
+size_t panel_doubles(int n) { return std::max((size_t)4 * GJ_WINDOW_MAX * n, sym_panel_doubles(n)); }
+
 // Device doubles of one slot sized for (Np, Nt): the chunk's Schur slots,
 // the W^-1 blocks, the R ping-pong buffers, the dipole rows, the asymptotic
 // window store and the inverse's panel windows (every piece 256-byte aligned).
@@ -1377,13 +1431,13 @@ size_t slot_doubles(const BatchDev& b, int Np, int Nt, int l_cont, bool keep_win
     const int nslots = b.N - b.n_s + 1;
     auto al = [](size_t c) { return (c + 31) & ~size_t(31); };
     const size_t np2 = (size_t)Np * Np, nt2 = (size_t)Nt * Nt;
-    const size_t base = 3 * al(SCHUR_CHUNK * np2) + al((size_t)Np * b.Nf) + al((size_t)b.Nf * b.Nf) +
-                        4 * al(nt2) + 2 * al((size_t)b.Krows * Nt) + al((size_t)SCHUR_CHUNK * 4 * GJ_WINDOW_MAX * Np) +
-                        al((size_t)4 * GJ_WINDOW_MAX * Nt);
+    const size_t base = 2 * al(SCHUR_CHUNK * np2) + al(SCHUR_CHUNK * al(sym_work_doubles(Np))) +
+                        al((size_t)Np * b.Nf) + al((size_t)b.Nf * b.Nf) + 3 * al(nt2) + al(sym_work_doubles(Nt)) +
+                        2 * al((size_t)b.Krows * Nt) + al(SCHUR_CHUNK * al(panel_doubles(Np))) + al(panel_doubles(Nt));
     if (keep_window) return base + al((size_t)nslots * nt2) + 2 * al((size_t)nslots * np2);
     return base + 2 * al((size_t)2 * Np * Nt) + al((size_t)b.nfit * 2 * Np) + al((size_t)8 * (l_cont + 1));
 }
-size_t slot_ints(int Np, int Nt) { return SCHUR_CHUNK * (6 * (size_t)Np + 4) + 6 * (size_t)Nt + 4; }
+size_t slot_ints(int Np, int Nt) { return SCHUR_CHUNK * (6 * (size_t)Np + 8) + 6 * (size_t)Nt; }
 // Device doubles of one group's chunk arrays (V, B, Bs, D^-1 of SCHUR_CHUNK steps, V(n+1) diagonal).
 size_t group_doubles(const BatchDev& b) {
     auto al = [](size_t c) { return (c + 31) & ~size_t(31); };
@@ -1456,6 +1510,9 @@ struct Scan {
     DevBuf<int> iarena, pia;
     DevBuf<GemmEntry> gm;
     DevBuf<GjEntry> gj;
+    DevBuf<SymEntry> sy;
+    DevBuf<unsigned long long> mag;
+    DevBuf<unsigned> barrier;
     VBAt vb;                            // V/B at one step for the post stages
     std::vector<PostBufs> P;            // gs energies
     std::vector<DevBuf<double>> keep;   // stability spectra per l_cont
@@ -1485,8 +1542,7 @@ int gemm_slots(Scan& sc, GemmEntry* ents, int count, int which, int opA, int opB
         case 0: M = Np; N = Np; break;       // S
         case 1: M = Np; N = Nf; break;       // T
         case 2: M = Nf; N = Nf; break;       // F
-        case 3: M = K; N = Np; break;        // G1
-        case 4: M = K; N = Nf; break;        // G2
+        case 3: M = K; N = std::max(Np, Nf); break;   // G1 and G2
         case 5: M = K; N = Nt; break;        // G3
         case 6: M = 2 * Np; N = Nt; break;   // GA (the fit accumulation)
     }
@@ -1529,6 +1585,8 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
     sc.nfit = sc.ne_fit - b.n_s + 1;
     b.count = slots;
     b.ngroups = ngroups;
+    b.sw_stride = (sym_work_doubles(sc.Np_cap) + 31) & ~size_t(31);
+    b.ps_stride = (panel_doubles(sc.Np_cap) + 31) & ~size_t(31);
     const int K = b.Krows, Nf = b.Nf;
     // ---- slot arena
     const bool keep = o.keep_window != 0;
@@ -1547,12 +1605,12 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
         // 256-byte aligned pieces (the inverse kernels copy 16-byte row pairs)
         auto take = [&p](size_t cnt) { double* r = p; p += (cnt + 31) & ~size_t(31); return r; };
         d.S = take(SCHUR_CHUNK * np2);
-        d.Sw = take(SCHUR_CHUNK * np2);
+        d.Sw = take(SCHUR_CHUNK * b.sw_stride);
         d.Sinv = take(SCHUR_CHUNK * np2);
         d.T = take((size_t)sc.Np_cap * Nf);
         d.F = take((size_t)Nf * Nf);
         d.Ra = take(nt2);
-        d.Rw = take(nt2);
+        d.Rw = take(sym_work_doubles(sc.Nt_cap));
         d.Rinv0 = take(nt2);
         d.Rinv1 = take(nt2);
         d.G0 = take((size_t)K * sc.Nt_cap);
@@ -1567,8 +1625,8 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
             d.wAB = take((size_t)b.nfit * 2 * sc.Np_cap);
             d.Mab = take((size_t)8 * (l_cap + 1));
         }
-        d.PS = take((size_t)SCHUR_CHUNK * 4 * GJ_WINDOW_MAX * sc.Np_cap);
-        d.PR = take((size_t)4 * GJ_WINDOW_MAX * sc.Nt_cap);
+        d.PS = take(SCHUR_CHUNK * b.ps_stride);
+        d.PR = take(panel_doubles(sc.Nt_cap));
         int* q = sc.iarena.p + slot_ints(sc.Np_cap, sc.Nt_cap) * e;
         const int Np = sc.Np_cap, Nt = sc.Nt_cap;
         d.sigS = q; q += SCHUR_CHUNK * Np;
@@ -1576,7 +1634,7 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
         d.sigR = q; q += Nt;
         d.ridR = q; q += Nt;
         d.stS = q; q += SCHUR_CHUNK * 4;
-        d.stR = q; q += 4;
+        d.stR = q; q += SCHUR_CHUNK * 4;
         d.sgS = q; q += SCHUR_CHUNK * 4 * Np;
         d.sgR = q; q += 4 * Nt;
         d.grp = e / sc.gs;
@@ -1607,13 +1665,18 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
     sc.start_chunk.assign(ngroups, 0);
     for (int g = 0; g < ngroups; ++g) sc.start_chunk[g] = (long)g * sc.chunks_per_sweep / ngroups;
     // ---- entry arrays
-    SCATT_TRY(sc.gm.alloc((6 + SCHUR_CHUNK) * (size_t)slots));
-    SCATT_TRY(sc.gj.alloc((1 + SCHUR_CHUNK) * (size_t)slots));
-    b.gmT = sc.gm.p; b.gmF = sc.gm.p + slots;
-    b.gmG1 = sc.gm.p + 2 * slots; b.gmG2 = sc.gm.p + 3 * slots; b.gmG3 = sc.gm.p + 4 * slots;
-    b.gmGA = sc.gm.p + 5 * slots;
-    b.gmS = sc.gm.p + 6 * slots;                   // SCHUR_CHUNK x slots
-    b.gjR = sc.gj.p; b.gjS = sc.gj.p + slots;      // gjS: SCHUR_CHUNK x slots
+    const size_t all = SCHUR_CHUNK * (size_t)slots;
+    SCATT_TRY(sc.gm.alloc(7 * all));
+    SCATT_TRY(sc.gj.alloc(2 * all));
+    SCATT_TRY(sc.sy.alloc(2 * all));
+    SCATT_TRY(sc.mag.alloc(8 * all));
+    SCATT_TRY(sc.barrier.alloc(SCHUR_CHUNK + 1));
+    b.gmS = sc.gm.p; b.gmT = sc.gm.p + all; b.gmF = sc.gm.p + 2 * all; b.gmG = sc.gm.p + 3 * all;
+    b.gmG3 = sc.gm.p + 5 * all; b.gmGA = sc.gm.p + 6 * all;
+    b.gjR = sc.gj.p; b.gjS = sc.gj.p + all;
+    b.syR = sc.sy.p; b.syS = sc.sy.p + all;
+    b.mag = sc.mag.p;
+    b.barrier = sc.barrier.p;
     // ---- post-stage buffers for one group
     SCATT_TRY(sc.vb.alloc(b));
     {
@@ -1726,6 +1789,9 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
     bool sweep[SCHUR_CHUNK] = {}, pts[SCHUR_CHUNK] = {}, win[SCHUR_CHUNK] = {};
     bool stab = false, stab_x = false, any_exch = false;
     const bool acc = sc.o.keep_window == 0;
+    // S and R are symmetric: the automatic scheme takes the symmetric sweep (half the flops, no
+    // column of pivots); the forced schemes keep the general inverse
+    const bool symmetric = g_inverse_scheme.load(std::memory_order_relaxed) == 0;
     int live_rinv[SCHUR_CHUNK] = {};
     std::vector<int> live_in(G, 0);
     for (int e = 0; e < count; ++e) live_in[sc.ed[e].grp] += sc.ed[e].live;
@@ -1752,43 +1818,46 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                               (sc.chunk % (sc.o.use_graphs ? 16 : 2) == 0);
     auto issue = [&]() -> int {
         // ---- Schur complements of the chunk's steps: A(n), S(n) = A - Bs B^T, one batched inverse
-        k_build_V<<<dim3(cdiv(b.n_pairs, TPB), G, SCHUR_CHUNK), TPB, 0, s>>>(b);
-        SCATT_COUNT_LAUNCH(1);
-        {
-            const int rows = std::max(b.Np_max * b.n_sigma, b.Nf);
-            k_build_B<<<dim3(cdiv(rows, 128), G, SCHUR_CHUNK), 128, 0, s>>>(b);
+        auto run = [&](auto kernel, dim3 grid, int threads, size_t smem, auto... args) -> int {
             SCATT_COUNT_LAUNCH(1);
-        }
-        k_init_S<<<dim3(64, count, SCHUR_CHUNK), TPB, 0, s>>>(b);
-        SCATT_COUNT_LAUNCH(1);
-        if (stab) { k_stab<<<dim3(count, SCHUR_CHUNK), TPB, 0, s>>>(b, 0); SCATT_COUNT_LAUNCH(1); }
-        k_prepare_schur<<<cdiv(count * SCHUR_CHUNK, 128), 128, 0, s>>>(b);
-        SCATT_COUNT_LAUNCH(1);
+            return cuda_status(launch_dep(kernel, grid, dim3(threads), smem, s, args...), "run_chunk");
+        };
+        SCATT_TRY(run(k_build_V, dim3(cdiv(b.n_pairs, TPB), G, SCHUR_CHUNK), TPB, 0, b));
+        SCATT_TRY(run(k_build_B, dim3(cdiv(std::max(b.Np_max * b.n_sigma, b.Nf), 128), G, SCHUR_CHUNK), 128, 0, b));
+        SCATT_TRY(run(k_init_S, dim3(64, count, SCHUR_CHUNK), TPB, 0, b));
+        if (stab) SCATT_TRY(run(k_stab, dim3(count, SCHUR_CHUNK), TPB, 0, b, 0));
+        SCATT_TRY(run(k_prepare, dim3(cdiv(count * SCHUR_CHUNK, 128)), 128, 0, b));
         if (any_exch) SCATT_TRY(gemm_slots(sc, b.gmS, count * SCHUR_CHUNK, 0, 0, 1));
-        if (stab_x) { k_stab<<<dim3(count, SCHUR_CHUNK), TPB, 0, s>>>(b, 1); SCATT_COUNT_LAUNCH(1); }
-        SCATT_TRY(gj_inverse_selected(b.gjS, count * SCHUR_CHUNK, sc.Np_cap, true, s, true));
+        if (stab_x) SCATT_TRY(run(k_stab, dim3(count, SCHUR_CHUNK), TPB, 0, b, 1));
+        if (symmetric) {
+            SCATT_TRY(sym_pack_batched(b.syS, count * SCHUR_CHUNK, sc.Np_cap, s));
+            SCATT_TRY(sym_sweep_batched(b.syS, count * SCHUR_CHUNK, sc.Np_cap, s));
+            SCATT_TRY(sym_rescue_batched(b.syS, count * SCHUR_CHUNK, b.barrier + SCHUR_CHUNK, s));
+        } else {
+            SCATT_TRY(gj_inverse_selected(b.gjS, count * SCHUR_CHUNK, sc.Np_cap, true, s, true));
+        }
         // ---- the R-ratio recurrence over the chunk's steps
         const dim3 eg(64, count);
         for (int j = 0; j < SCHUR_CHUNK; ++j) {
             if (!step[j]) continue;
-            k_prepare<<<cdiv(count, 128), 128, 0, s>>>(b, j);
-            SCATT_COUNT_LAUNCH(1);
-            if (start[j]) { k_vdiag<<<dim3(cdiv(b.Np_max, 128), G), 128, 0, s>>>(b, j); SCATT_COUNT_LAUNCH(1); }
-            k_collect<<<cdiv(count, 128), 128, 0, s>>>(b, j, 0);
-            SCATT_COUNT_LAUNCH(1);
+            const size_t at = (size_t)j * count;
+            if (start[j]) SCATT_TRY(run(k_vdiag, dim3(cdiv(b.Np_max, 128), G), 128, 0, b, j));
             if (exch[j]) {
-                SCATT_TRY(gemm_slots(sc, b.gmT, count, 1, 0, 0));
-                SCATT_TRY(gemm_slots(sc, b.gmF, count, 2, 1, 0));
+                SCATT_TRY(gemm_slots(sc, b.gmT + at, count, 1, 0, 0));
+                SCATT_TRY(gemm_slots(sc, b.gmF + at, count, 2, 1, 0));
             }
             if (start[j]) {
-                k_analytic_R<<<eg, TPB, 0, s>>>(b, j);
-                SCATT_COUNT_LAUNCH(1);
-                k_analytic_R_diag<<<dim3(4, count), TPB, 0, s>>>(b, j);
-                SCATT_COUNT_LAUNCH(1);
+                SCATT_TRY(run(k_analytic_R, eg, TPB, 0, b, j));
+                SCATT_TRY(run(k_analytic_R_diag, dim3(4, count), TPB, 0, b, j));
             }
             if (rinv[j]) {
-                k_assemble_R<<<eg, TPB, 0, s>>>(b, j);
-                SCATT_COUNT_LAUNCH(1);
+                if (symmetric) {
+                    const int T = sym_tiles_of(sc.Nt_cap);
+                    SCATT_TRY(run(k_assemble_R_tiles, dim3(T * (T + 1) / 2, count), SYM_THREADS, sizeof(SymDiagShared),
+                                  b, j));
+                } else {
+                    SCATT_TRY(run(k_assemble_R, eg, TPB, 0, b, j));
+                }
                 const bool sample = sample_chunk && j == 0;
                 cudaEvent_t a0 = nullptr, a1 = nullptr;
                 if (sample) {
@@ -1796,7 +1865,12 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                     SCATT_TRY(sc.events.get(&a1));
                     SCATT_CUDA_TRY(cudaEventRecord(a0, s));
                 }
-                SCATT_TRY(gj_inverse_selected(b.gjR, count, sc.Nt_cap, true, s, true));
+                if (symmetric) {
+                    SCATT_TRY(sym_sweep_batched(b.syR + at, count, sc.Nt_cap, s));
+                    SCATT_TRY(sym_rescue_launch(b.syR + at, count, b.barrier + j, RSource{b, j}, s));
+                } else {
+                    SCATT_TRY(gj_inverse_selected(b.gjR + at, count, sc.Nt_cap, true, s, true));
+                }
                 if (sample) {
                     SCATT_CUDA_TRY(cudaEventRecord(a1, s));
                     tm->rinv.push_back({a0, a1});
@@ -1807,25 +1881,22 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                         tm->flops += 2.0 * n * n * n;
                     }
                 }
-                k_collect<<<cdiv(count, 128), 128, 0, s>>>(b, j, 1);
-                SCATT_COUNT_LAUNCH(1);
             }
             if (sweep[j]) {
-                if (pts[j]) SCATT_TRY(gemm_slots(sc, b.gmG1, count, 3, 0, 0));
-                if (pts[j] && exch[j]) SCATT_TRY(gemm_slots(sc, b.gmG2, count, 4, 0, 0));
-                SCATT_TRY(gemm_slots(sc, b.gmG3, count, 5, 0, 0));
+                // C_n Sinv and -C_n T go to different columns of G(n-1)^T: one batch
+                if (pts[j]) SCATT_TRY(gemm_slots(sc, b.gmG + 2 * at, exch[j] ? 2 * count : count, 3, 0, 0));
+                SCATT_TRY(gemm_slots(sc, b.gmG3 + at, count, 5, 0, 0));
             }
             if (win[j]) {
-                k_acc_ab<<<eg, TPB, 0, s>>>(b, j);
-                SCATT_COUNT_LAUNCH(1);
-                SCATT_TRY(gemm_slots(sc, b.gmGA, count, 6, 0, 0));
+                SCATT_TRY(run(k_acc_ab, eg, TPB, 0, b, j));
+                SCATT_TRY(gemm_slots(sc, b.gmGA + at, count, 6, 0, 0));
             }
         }
-        k_advance<<<1, MAX_GROUPS, 0, s>>>(b);
-        SCATT_COUNT_LAUNCH(1);
+        SCATT_TRY(run(k_collect, dim3(cdiv(count, 128)), 128, 0, b));
+        SCATT_TRY(run(k_advance, dim3(1), MAX_GROUPS, 0, b));
         return SCATT_CUDA_TRY_RET(cudaGetLastError());
     };
-    uint64_t key = (stab ? 1u : 0u) | (stab_x ? 2u : 0u) | (any_exch ? 4u : 0u);
+    uint64_t key = (stab ? 1u : 0u) | (stab_x ? 2u : 0u) | (any_exch ? 4u : 0u) | ((uint64_t)symmetric << 59);
     for (int j = 0; j < SCHUR_CHUNK; ++j) {
         const uint64_t bits = (step[j] ? 1u : 0u) | (exch[j] ? 2u : 0u) | (start[j] ? 4u : 0u) |
                               (rinv[j] ? 8u : 0u) | (sweep[j] ? 16u : 0u) | (pts[j] ? 32u : 0u) |

@@ -9,6 +9,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "sym_tiles.cuh"
 
 namespace scatt {
 
@@ -56,7 +57,7 @@ struct EnergyDev {
     double *tailR, *tailS, *psiT;
     int *sigS, *ridS, *stS;   // SCHUR_CHUNK slots (Np, Np, 4 ints each)
     int *sigR, *ridR, *stR;
-    double *PS, *PR;       // two-level panel windows (4 x Np x 64 per Schur slot, 4 x Nt x 64)
+    double *PS, *PR;       // inverse panels: ps_stride doubles per Schur slot, one R panel
     int *sgS, *sgR;        // composite row maps of the windows (4 x Np per Schur slot, 4 x Nt)
     // forward accumulation of the amplitude fit (no window store: tailR == nullptr):
     // GA0 / GA1 (2 Np x N_t, ld 2 Np) hold G_A(n-1)^T by parity, with
@@ -90,9 +91,15 @@ struct BatchDev {
     const int* l_of_mu;
     const int* l_sigma;
     GroupDev* grp;          // ngroups entries
-    // entry arrays written by k_prepare
-    GemmEntry *gmS, *gmT, *gmF, *gmG1, *gmG2, *gmG3, *gmGA;
+    // entry arrays written by k_prepare, SCHUR_CHUNK x slots each
+    GemmEntry *gmS, *gmT, *gmF, *gmG, *gmG3, *gmGA;   // gmG: per step all C_n Sinv, then all -C_n T
     GjEntry *gjS, *gjR;
+    // the same inverses for the symmetric sweep, their magnitudes (4 words
+    // each), and the rescue's barrier counters: one per step's R, one for S
+    SymEntry *syS, *syR;
+    unsigned long long* mag;
+    unsigned* barrier;
+    size_t sw_stride, ps_stride;    // doubles of one Schur slot in Sw and PS
     EnergyDev* ed;
 };
 

@@ -1,0 +1,291 @@
+// sym_rescue.cuh -- what follows a symmetric sweep whose intermediate
+// inverses grew (see sym_inverse.cu): one launch per batch, which returns at
+// once when no entry needs it.
+//
+// A sweep's error grows with g, the larger of max|D| / max|A^-1| and of the
+// Schur complements' largest element over A's, and with max|A| max|D| where A
+// holds one dominant direction that every tile has a part of.  The inverse
+// takes a Newton step X <- X (2 I - A X), two products over the whole grid
+// for that entry alone, which squares the relative error, where g > 3 or
+// max|A| max|D| > 3e3 (about 1 in 30 matrices of a radial sweep at a step of
+// 0.05 bohr, and fewer the finer the grid), and a second one above g = 1e3.
+// Measured on the matrices of one sweep (order 1046, kappa = max|A| max|X|),
+// relative errors:
+//              g       kappa   sweep    Newton   LU       Gauss-Jordan, pivoted
+//              1200    21      3.9e-11  7.7e-16  8.4e-16  1.1e-14
+//              0.94    2.1e6   3.1e-9   8.2e-13  1.9e-12  2.7e-13
+//              15      1.4e3   7.7e-13  7.0e-15  3.9e-13  7.4e-13
+//   median     1       20      7e-16             6e-16
+// Past g = 1e6, and on zero and non-finite pivots, to report them, the entry
+// takes a pivoted elimination by one CTA: slow, and not met in normal running.
+#pragma once
+
+#include "sym_tiles.cuh"
+
+namespace scatt {
+
+// Barrier over the grid's CTAs, all resident (cooperative launch): `turn`
+// counts the barriers passed on this counter, which starts at zero.  The wait
+// is bounded (about 10 s); false: it ran out.
+__device__ __forceinline__ bool sym_grid_barrier(unsigned* counter, unsigned& turn) {
+    __shared__ int s_ok;
+    __syncthreads();
+    ++turn;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(counter, 1u);
+        const unsigned want = turn * gridDim.x;
+        int ok = 0;
+        for (unsigned spin = 0; spin < (1u << 26); ++spin) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+            if (v >= want) { ok = 1; break; }
+            __nanosleep(100);
+        }
+        __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// Tile (i, j) of alpha A^T B, all of order n and column-major (A^T read by
+// columns of A); the 64 x 64 result in the accumulator layout of sym_tile_mma.
+__device__ __forceinline__ void sym_product_tile(double (&acc)[4][4], const double* A, int lda, const double* B,
+                                                 int ldb, int n, int i, int j, double* smem) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double *As = smem, *Bs = smem + SYM_TILE;
+#pragma unroll
+    for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) acc[nb][v] = 0.0;
+    for (int kb = 0; kb < n; kb += SYM_NB) {
+        __syncthreads();
+#pragma unroll 4
+        for (int u = 0; u < 16; ++u) {
+            const int x = warp * 8 + (u >> 1), k = lane + 32 * (u & 1), gk = kb + k;
+            const int ra = i * SYM_NB + x, rb = j * SYM_NB + x;
+            As[sym_pos(x, k)] = (ra < n && gk < n) ? A[gk + (size_t)ra * lda] : 0.0;
+            Bs[sym_pos(x, k)] = (rb < n && gk < n) ? B[gk + (size_t)rb * ldb] : 0.0;
+        }
+        __syncthreads();
+        sym_tile_mma(acc, As, Bs, warp & 3, warp >> 2, lane, 0, 8);
+    }
+}
+
+struct SymPivotShared {
+    unsigned long long best[32];
+    int row[32];
+    int p, stop;
+};
+
+// Gauss-Jordan elimination with partial pivoting of e.A by one CTA (rows stay
+// in place, as in sym_diag_invert; the pivot row and column go through e.W)
+// into e.out, symmetrised; e.status gets the first zero or non-finite pivot.
+__device__ __forceinline__ void sym_pivoted(const SymEntry& e, SymPivotShared& sh) {
+    const int n = e.n, tid = threadIdx.x;
+    double* A = e.A;
+    double* row = e.W;                // n doubles
+    double* col = e.W + n;            // n doubles
+    double* X = e.out;
+    // step of each row's pivot (-1: unused) and row of each step
+    double* step_of_row = reinterpret_cast<double*>(e.M);
+    double* row_of_step = reinterpret_cast<double*>(e.P);
+    for (int r = tid; r < n; r += blockDim.x) step_of_row[r] = -1.0;
+    if (tid == 0) sh.stop = 0;
+    __syncthreads();
+    for (int k = 0; k < n; ++k) {
+        unsigned long long b = 0;
+        int br = n;
+        for (int r = tid; r < n; r += blockDim.x) {
+            const double v = A[r + (size_t)k * n];
+            col[r] = v;
+            if (step_of_row[r] < 0.0) {
+                const unsigned long long key = sym_bits(v);
+                if (br == n || key > b) { b = key; br = r; }
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long ob = __shfl_xor_sync(0xffffffffu, b, o);
+            const int orow = __shfl_xor_sync(0xffffffffu, br, o);
+            if (orow < n && (br == n || ob > b || (ob == b && orow < br))) { b = ob; br = orow; }
+        }
+        if ((tid & 31) == 0) { sh.best[tid >> 5] = b; sh.row[tid >> 5] = br; }
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
+                if (sh.row[w] < n && (br == n || sh.best[w] > b || (sh.best[w] == b && sh.row[w] < br))) {
+                    b = sh.best[w];
+                    br = sh.row[w];
+                }
+            sh.p = br;
+            const double v = __longlong_as_double((long long)b);
+            if (!isfinite(v) || v == 0.0) {
+                e.status[0] = isfinite(v) ? DEV_SINGULAR : DEV_NONFINITE;
+                e.status[1] = k;
+                sh.stop = 1;
+            }
+            step_of_row[br] = k;
+            row_of_step[k] = br;
+        }
+        __syncthreads();
+        if (sh.stop) break;
+        const int p = sh.p;
+        for (int c = tid; c < n; c += blockDim.x) row[c] = A[p + (size_t)c * n];
+        __syncthreads();
+        const double rp = 1.0 / col[p];
+        for (long u = tid; u < (long)n * n; u += blockDim.x) {
+            const int r = (int)(u % n), c = (int)(u / n);
+            double v;
+            if (r == p) v = c == k ? rp : row[c] * rp;
+            else v = c == k ? -col[r] * rp : A[u] - (col[r] * rp) * row[c];
+            A[u] = v;
+        }
+        __syncthreads();
+    }
+    if (sh.stop) {
+        const double bad = __longlong_as_double(0x7ff8000000000000ll);
+        for (long u = tid; u < (long)n * n; u += blockDim.x) X[(u % n) + (size_t)(u / n) * e.ldo] = bad;
+        return;
+    }
+    // A[p_k][j] = inv[k][p_j]
+    for (long u = tid; u < (long)n * n; u += blockDim.x) {
+        const int r = (int)(u % n), c = (int)(u / n);
+        X[(int)step_of_row[r] + (size_t)(int)row_of_step[c] * e.ldo] = A[u];
+    }
+    __syncthreads();
+    for (long u = tid; u < (long)n * n; u += blockDim.x) {
+        const int r = (int)(u % n), c = (int)(u / n);
+        if (c >= r) continue;
+        const double v = 0.5 * (X[r + (size_t)c * e.ldo] + X[c + (size_t)r * e.ldo]);
+        X[r + (size_t)c * e.ldo] = v;
+        X[c + (size_t)r * e.ldo] = v;
+    }
+}
+
+constexpr int SYM_RESCUE_LIST = 256;          // entries looked at in one pass
+
+// `source` fills rows and columns of entry.A from what the caller still has
+// (index, entry, first element, stride); entry.A may also have been kept.
+template <class Source>
+__global__ void __launch_bounds__(SYM_THREADS, 1)
+sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, Source source) {
+    extern __shared__ double smem[];
+    __shared__ int s_mode[SYM_RESCUE_LIST];
+    __shared__ SymPivotShared s_piv;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wr = warp & 3, wc = warp >> 2, g = lane >> 2, t = lane & 3;
+    unsigned turn = 0;
+    bool alive = true;
+    for (int base = 0; base < count; base += SYM_RESCUE_LIST) {
+        const int m = min(SYM_RESCUE_LIST, count - base);
+        int any = 0;
+        for (int k = tid; k < m; k += SYM_THREADS) {
+            const SymEntry& e = entries[base + k];
+            int mode = 0;
+            if (e.n > 0) {
+                const double d = __longlong_as_double((long long)e.mag[0]);
+                const double x = __longlong_as_double((long long)e.mag[1]);
+                const double a = __hiloint2double((int)*sym_hi_of_A(e), 0), s = __hiloint2double((int)*sym_hi_of_schur(e), 0);
+                const double gr = fmax(d / x, s / a);
+                if (!isfinite(d) || !isfinite(x) || !isfinite(a) || !(x > 0.0) || !(gr <= 1e6)) mode = 3;
+                else if (gr > 1e3) mode = 2;
+                else if (gr > 3.0 || a * d > 3e3) mode = 1;
+                if (blockIdx.x == 0) {
+                    e.mag[3] = (unsigned long long)mode;
+                    e.status[0] = 0;
+                    e.status[1] = 0;
+                }
+            }
+            s_mode[k] = mode;
+            any |= mode;
+        }
+        if (!__syncthreads_or(any)) continue;
+        // Newton steps, entry by entry over the whole grid
+        for (int k = 0; k < m && alive; ++k) {
+            const int mode = s_mode[k];
+            if (mode != 1 && mode != 2) continue;
+            const SymEntry e = entries[base + k];
+            const int n = e.n, T = sym_tiles_of(n);
+            source(base + k, e, blockIdx.x * SYM_THREADS + tid, gridDim.x * SYM_THREADS);
+            alive = sym_grid_barrier(barrier, turn);
+            for (int step = 0; step < mode && alive; ++step) {
+                for (int half = 0; half < 2 && alive; ++half) {
+                    // W = A X, then the second half of W = X W (A and X are symmetric)
+                    for (int u = blockIdx.x; u < T * T; u += gridDim.x) {
+                        const int i = u % T, j = u / T;
+                        double acc[4][4];
+                        if (half == 0) sym_product_tile(acc, e.A, n, e.out, e.ldo, n, i, j, smem);
+                        else sym_product_tile(acc, e.out, e.ldo, e.W, n, n, i, j, smem);
+                        double* C = half == 0 ? e.W : e.W + (size_t)n * n;
+#pragma unroll
+                        for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+                            for (int v = 0; v < 4; ++v) {
+                                const int r = i * SYM_NB + wr * 16 + g + ((v >> 1) << 3);
+                                const int c = j * SYM_NB + wc * 32 + nb * 8 + 2 * t + (v & 1);
+                                if (r < n && c < n) C[r + (size_t)c * n] = acc[nb][v];
+                            }
+                    }
+                    alive = sym_grid_barrier(barrier, turn);
+                }
+                if (!alive) break;
+                const double* Z = e.W + (size_t)n * n;
+                for (long u = blockIdx.x * (long)SYM_THREADS + tid; u < (long)n * n; u += (long)gridDim.x * SYM_THREADS) {
+                    const int r = (int)(u % n), c = (int)(u / n);
+                    if (c > r) continue;
+                    const double z = 0.5 * (Z[r + (size_t)c * n] + Z[c + (size_t)r * n]);
+                    const double x = 2.0 * e.out[r + (size_t)c * e.ldo] - z;
+                    e.out[r + (size_t)c * e.ldo] = x;
+                    e.out[c + (size_t)r * e.ldo] = x;
+                }
+                alive = sym_grid_barrier(barrier, turn);
+            }
+            if (!alive && blockIdx.x == 0 && tid == 0) e.status[0] = DEV_NONFINITE;
+        }
+        // pivoted eliminations, one CTA each
+        for (int k = 0; k < m; ++k) {
+            if (s_mode[k] != 3 || (base + k) % (int)gridDim.x != (int)blockIdx.x) continue;
+            const SymEntry e = entries[base + k];
+            source(base + k, e, tid, SYM_THREADS);
+            __syncthreads();
+            sym_pivoted(e, s_piv);
+            __syncthreads();
+        }
+        __syncthreads();                        // s_mode is rewritten
+    }
+}
+
+template <class Source>
+int sym_rescue_launch(const SymEntry* entries_dev, int count, unsigned* barrier, Source source, cudaStream_t stream) {
+    if (count <= 0) return SCATT_OK;
+    int dev = 0, sms = 0;
+    SCATT_CUDA_TRY(cudaGetDevice(&dev));
+    static std::atomic<int> grid_of[64];
+    const size_t smem = 2 * SYM_TILE * sizeof(double);
+    sms = dev >= 0 && dev < 64 ? grid_of[dev].load() : 0;
+    if (sms == 0) {
+        SCATT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        SCATT_CUDA_TRY(cudaFuncSetAttribute(sym_rescue_kernel<Source>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)smem));
+        if (dev >= 0 && dev < 64) grid_of[dev].store(sms);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sms);
+    cfg.blockDim = dim3(SYM_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    SCATT_CUDA_TRY(cudaLaunchKernelEx(&cfg, sym_rescue_kernel<Source>, entries_dev, count, barrier, source));
+    SCATT_COUNT_LAUNCH(1);
+    return SCATT_OK;
+}
+
+// For callers whose entry.A is intact; barrier: one zeroed word.
+int sym_rescue_batched(const SymEntry* entries_dev, int count, unsigned* barrier, cudaStream_t stream);
+
+}  // namespace scatt

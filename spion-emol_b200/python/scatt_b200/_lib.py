@@ -59,6 +59,7 @@ def lib():
         getattr(L, f).argtypes = [C.c_int, C.c_double]
     L.scatt_inverse_batched.argtypes = [C.c_int, C.c_int, dptr, dptr, C.c_int, iptr]
     L.scatt_inverse_batched_noalloc.argtypes = [C.c_int, C.c_int, dptr, dptr, C.c_int, iptr]
+    L.scatt_inverse_symmetric_batched.argtypes = [C.c_int, C.c_int, dptr, dptr, iptr, iptr]
     L.scatt_dgemm.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_double,
                               dptr, C.c_int, dptr, C.c_int, C.c_double, dptr, C.c_int]
     L.scatt_bench_inverse.argtypes = [C.c_int, C.c_int, C.c_int, dptr]
@@ -113,6 +114,19 @@ def inverse_batched(A: np.ndarray, symmetrize: bool = False, noalloc: bool = Fal
     if code not in (0, 4, 5):
         check(code)
     return (inv[0] if single else inv), st
+
+
+def inverse_symmetric_batched(A: np.ndarray):
+    """Inverses of the symmetric matrices A (count, n, n); returns (inv,
+    status, mode) (scatt_inverse_symmetric_batched)."""
+    A = np.ascontiguousarray(A, dtype=np.float64)
+    count, n, _ = A.shape
+    out = np.empty_like(A)
+    st, mode = np.zeros((count, 2), dtype=np.int32), np.zeros(count, dtype=np.int32)
+    code = lib().scatt_inverse_symmetric_batched(n, count, as_dptr(A), as_dptr(out), as_iptr(st), as_iptr(mode))
+    if code not in (0, 4, 5):
+        check(code)
+    return out, st, mode
 
 
 def dgemm(A, B, C=None, alpha=1.0, beta=0.0, opA=0, opB=0):

@@ -1,0 +1,73 @@
+"""The symmetric sweep inverse against numpy: tile edges, orders past one
+tile, indefinite matrices, and matrices whose leading block is (nearly)
+singular although they are not, which need Newton steps or the pivoted
+elimination."""
+import numpy as np
+import pytest
+
+from scatt_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def symmetric(rng, count, n):
+    """Indefinite, kappa of a few tens: a scaled random symmetric part (norm
+    about 0.9) on a diagonal of 2 with every fifth sign turned."""
+    M = rng.standard_normal((count, n, n))
+    M = (M + np.swapaxes(M, 1, 2)) * (0.9 / (2.0 * np.sqrt(2.0 * n)))
+    M[:, np.arange(n), np.arange(n)] += np.where(np.arange(n) % 5 == 0, -2.0, 2.0)
+    return M
+
+
+@pytest.mark.parametrize("n,count", [(1, 3), (2, 1), (17, 5), (63, 2), (64, 2), (65, 3), (100, 20), (127, 1), (128, 2),
+                                     (129, 1), (162, 4), (193, 2), (324, 3), (441, 9), (774, 2), (1046, 2), (1314, 1)])
+def test_matches_numpy(n, count):
+    A = symmetric(np.random.default_rng(n), count, n)
+    X, st, mode = _lib.inverse_symmetric_batched(A)
+    assert np.all(st == 0) and np.all(mode == 0)
+    assert np.array_equal(X, np.swapaxes(X, 1, 2))
+    for a, x in zip(A, X):
+        ref = np.linalg.inv(a)
+        # kappa <= 2.9 / 1.1 up to the random part's spread: rounding of n-term sums, with room for growth below 10
+        assert np.max(np.abs(x - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+def test_pivots_inside_a_tile():
+    n = 64
+    A = np.zeros((1, n, n))
+    i = np.arange(0, n, 2)
+    A[0, i, i + 1] = A[0, i + 1, i] = 1.0 + i / n          # zero diagonal: 2 x 2 pivots only
+    X, st, mode = _lib.inverse_symmetric_batched(A)
+    assert st[0, 0] == 0 and mode[0] == 0
+    assert np.max(np.abs(X[0] @ A[0] - np.eye(n))) <= 1e-15
+
+
+@pytest.mark.parametrize("n", [128, 200, 450])
+@pytest.mark.parametrize("delta,want", [(0.02, 1), (2e-3, 1), (1e-5, 2), (0.0, 3)])
+def test_nearly_singular_leading_block(n, delta, want):
+    """[[delta I, I], [I, A22]] on the first two tiles: |D| of the first pivot
+    tile is 1 / delta, |X| about 2.  The sweep's error is delta^-2 eps (up to
+    6e-11 and 2e-6); one Newton step, or two, square it away, leaving
+    rounding; delta = 0 leaves no first pivot at all."""
+    rng = np.random.default_rng(5)
+    A = symmetric(rng, 2, n)
+    A[1, :64, :64] = delta * np.eye(64)
+    A[1, :64, 64:128] = A[1, 64:128, :64] = np.eye(64)
+    A[1, :64, 128:] = A[1, 128:, :64] = 0.0
+    X, st, mode = _lib.inverse_symmetric_batched(A)
+    assert np.all(st[:, 0] == 0) and mode[0] == 0 and mode[1] == want
+    for a, x in zip(A, X):
+        ref = np.linalg.inv(a)
+        kappa = np.linalg.cond(a)
+        assert np.max(np.abs(x - ref)) <= 1e-13 * max(10.0, kappa) * np.max(np.abs(ref))
+        assert np.array_equal(x, x.T)
+
+
+def test_singular_and_nonfinite_are_reported():
+    A = symmetric(np.random.default_rng(1), 3, 100)
+    A[0, 70, :] = A[0, :, 70] = 0.0
+    A[2, 5, 5] = np.nan
+    X, st, mode = _lib.inverse_symmetric_batched(A)
+    assert st[0, 0] == 1 and st[1, 0] == 0 and st[2, 0] == 2
+    ref = np.linalg.inv(A[1])
+    assert np.max(np.abs(X[1] - ref)) <= 1e-12 * np.max(np.abs(ref))
