@@ -6,8 +6,8 @@
 // lower triangle) and (b) the eigenphases atan(eig K) of
 // KMatrixExtractor.cpp:185-191 / AsymptoticAmplitudes.cpp:340-344.
 //
-// Method: Householder reduction to tridiagonal form (one CTA per matrix,
-// reading only the lower triangle, in place in global memory), then
+// Method: Householder reduction to tridiagonal form (one cluster of CTAs per
+// matrix, reading only the lower triangle, in place in global memory), then
 // Sturm-sequence bisection for the requested eigenvalues.  Both steps are
 // backward stable, so eigenvalues are accurate to O(eps ||M||), the same
 // guarantee the reference's QR-based solver gives.
@@ -22,6 +22,7 @@ namespace {
 
 constexpr int ET = 256;
 
+// Sum over the CTA, the same value (and bits) in every thread.
 __device__ double block_sum(double v, double* red) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -29,143 +30,184 @@ __device__ double block_sum(double v, double* red) {
     if (lane == 0) red[w] = v;
     __syncthreads();
     double s = 0.0;
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < ET / 32; ++i) s += red[i];
-        red[ET / 32] = s;
-    }
-    __syncthreads();
-    return red[ET / 32];
+#pragma unroll
+    for (int i = 0; i < ET / 32; ++i) s += red[i];
+    return s;
 }
 
-// Sturm count: number of eigenvalues of the tridiagonal (d, e) below x.
-__device__ int sturm_count(const double* d, const double* e, int n, double x) {
+// One matrix on a cluster of EC CTAs, in place in global memory (it stays in
+// L2).  Columns are dealt to the cluster's warps; every CTA forms the
+// Householder vector of each step itself.  A step's rank-2 update is applied
+// in the next step's pass over the matrix, which also forms that step's
+// product A v, so that the trailing matrix is passed once and the cluster
+// meets once per step (to exchange p = beta A v, double-buffered in the work
+// array); the one column that the others read next is not written in that
+// pass.  Bound by the chain of n steps, each a few L2 latencies: order 441,
+// 99.3 ms with one CTA per matrix, two passes and a matrix-vector product of
+// one row per thread.
+constexpr int EC = 8;
+
+__global__ void __cluster_dims__(EC, 1, 1) __launch_bounds__(ET)
+tridiag_kernel(const EigEntry* entries) {
+    const EigEntry en = entries[blockIdx.x / EC];
+    const int n = en.n, ld = en.ld;
+    double* M = en.M;
+    double *d = en.d, *e = en.e;
+    extern __shared__ double esm[];
+    double* v = esm;              // Householder vector of the last step, rows below it
+    double* w = esm + n;          // its partner in the pending update A -= v w^T + w v^T
+    double* x = esm + 2 * n;      // vector of this step
+    __shared__ double red[ET / 32];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int rank = blockIdx.x % EC, gw = rank * (ET / 32) + (tid >> 5);
+    constexpr int GW = EC * ET / 32;
+    auto meet = [] {
+        asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    };
+    // only the lower triangle is read: mirror it into the upper triangle first
+    for (int j = gw; j < n; j += GW)
+        for (int i = j + 1 + lane; i < n; i += 32) M[j + (size_t)i * ld] = M[i + (size_t)j * ld];
+    for (int i = tid; i < n; i += ET) v[i] = w[i] = 0.0;
+    meet();
+    for (int k = 0; k + 2 < n; ++k) {
+        // column k with the pending update: x below the diagonal
+        const double vk = v[k], wk = w[k];
+        double ss = 0.0;
+        for (int i = k + 1 + tid; i < n; i += ET) {
+            const double c = __ldcg(&M[i + (size_t)k * ld]) - (v[i] * wk + w[i] * vk);
+            x[i] = c;
+            ss += c * c;
+        }
+        const double nrm2 = block_sum(ss, red);
+        const double x0 = x[k + 1];
+        double alpha = x0 > 0.0 ? -sqrt(nrm2) : sqrt(nrm2), beta = 0.0;    // beta = 2 / (v^T v)
+        if (nrm2 > 0.0) {
+            const double vtv = nrm2 - x0 * x0 + (x0 - alpha) * (x0 - alpha);
+            beta = vtv > 0.0 ? 2.0 / vtv : 0.0;
+        } else {
+            alpha = 0.0;
+        }
+        if (rank == 0 && tid == 0) {
+            d[k] = __ldcg(&M[k + (size_t)k * ld]) - 2.0 * vk * wk;
+            e[k] = alpha;
+        }
+        __syncthreads();                           // every thread has read x[k + 1]
+        if (tid == 0) x[k + 1] = x0 - alpha;
+        __syncthreads();
+        // pending update and p = beta A x on this warp's columns
+        double* p = en.work + (size_t)(k & 1) * n;
+        for (int j = k + 1 + gw; j < n; j += GW) {
+            double* col = M + (size_t)j * ld;
+            const double vj = v[j], wj = w[j];
+            double s = 0.0;
+            for (int i = k + 1 + lane; i < n; i += 32) {
+                const double c = col[i] - (v[i] * wj + w[i] * vj);
+                col[i] = c;
+                s += c * x[i];
+            }
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+            if (lane == 0) p[j] = beta * s;
+        }
+        meet();
+        // w = p - (beta / 2) (p^T x) x; x becomes v
+        double pv = 0.0;
+        for (int i = k + 1 + tid; i < n; i += ET) {
+            const double c = __ldcg(&p[i]);
+            w[i] = c;
+            pv += c * x[i];
+        }
+        const double K = 0.5 * beta * block_sum(pv, red);
+        for (int i = k + 1 + tid; i < n; i += ET) {
+            w[i] = beta == 0.0 ? 0.0 : w[i] - K * x[i];
+            v[i] = x[i];
+        }
+        __syncthreads();
+    }
+    if (rank == 0 && tid == 0) {
+        auto at = [&](int i, int j) { return __ldcg(&M[i + (size_t)j * ld]) - (v[i] * w[j] + w[i] * v[j]); };
+        if (n >= 2) {
+            d[n - 2] = at(n - 2, n - 2);
+            e[n - 2] = at(n - 1, n - 2);
+        }
+        d[n - 1] = at(n - 1, n - 1);
+    }
+    meet();                                        // no CTA leaves while another may still read its columns
+}
+
+// Sturm count: number of eigenvalues of the tridiagonal (d, e^2) below x.
+__device__ int sturm_count(const double* d, const double* e2, int n, double x) {
     int cnt = 0;
     double q = d[0] - x;
     if (q < 0.0) ++cnt;
     for (int i = 1; i < n; ++i) {
         if (q == 0.0) q = 1e-300;
-        q = (d[i] - x) - e[i - 1] * e[i - 1] / q;
+        q = (d[i] - x) - e2[i - 1] / q;
         if (q < 0.0) ++cnt;
     }
     return cnt;
 }
 
-__device__ double bisect_kth(const double* d, const double* e, int n, int kth, double lo, double hi) {
+__device__ double bisect_kth(const double* d, const double* e2, int n, int kth, double lo, double hi) {
     // smallest x with count(x) > kth
     for (int it = 0; it < 200; ++it) {
         const double mid = 0.5 * (lo + hi);
         if (mid <= lo || mid >= hi) break;
-        if (sturm_count(d, e, n, mid) > kth) hi = mid; else lo = mid;
+        if (sturm_count(d, e2, n, mid) > kth) hi = mid; else lo = mid;
     }
     return 0.5 * (lo + hi);
 }
 
-__global__ void __launch_bounds__(ET)
-tridiag_kernel(const EigEntry* __restrict__ entries) {
-    const EigEntry en = entries[blockIdx.x];
-    const int n = en.n;
-    double* M = en.M;
-    const int ld = en.ld;
-    double* d = en.d;
-    double* e = en.e;
-    double* v = en.work;          // n
-    double* p = en.work + n;      // n
-    __shared__ double red[ET / 32 + 1];
-    __shared__ double s_alpha, s_beta;
-    const int tid = threadIdx.x;
-    // only the lower triangle is read: mirror it into the upper triangle first
-    for (int j = 0; j < n; ++j)
-        for (int i = j + 1 + tid; i < n; i += ET) M[j + (size_t)i * ld] = M[i + (size_t)j * ld];
-    __syncthreads();
-    for (int k = 0; k + 2 < n; ++k) {
-        // x = M[k+1:n, k]
-        double ss = 0.0;
-        for (int i = k + 1 + tid; i < n; i += ET) {
-            const double x = M[i + (size_t)k * ld];
-            ss += x * x;
-        }
-        const double nrm2 = block_sum(ss, red);
-        if (tid == 0) {
-            const double x0 = M[(k + 1) + (size_t)k * ld];
-            const double nrm = sqrt(nrm2);
-            double alpha = (x0 > 0.0) ? -nrm : nrm;
-            double beta = 0.0;                      // 2 / (v^T v)
-            if (nrm2 > 0.0) {
-                const double vtv = nrm2 - x0 * x0 + (x0 - alpha) * (x0 - alpha);
-                beta = vtv > 0.0 ? 2.0 / vtv : 0.0;
-            } else {
-                alpha = 0.0;
-            }
-            s_alpha = alpha;
-            s_beta = beta;
-            d[k] = M[k + (size_t)k * ld];
-            e[k] = alpha;
-        }
-        __syncthreads();
-        const double alpha = s_alpha, beta = s_beta;
-        for (int i = k + 1 + tid; i < n; i += ET) {
-            double x = M[i + (size_t)k * ld];
-            if (i == k + 1) x -= alpha;
-            v[i] = x;
-        }
-        __syncthreads();
-        if (beta == 0.0) continue;
-        // p = beta * A_sub v
-        for (int i = k + 1 + tid; i < n; i += ET) {
-            double s = 0.0;
-            for (int j = k + 1; j < n; ++j) s += M[i + (size_t)j * ld] * v[j];
-            p[i] = beta * s;
-        }
-        __syncthreads();
-        // w = p - (beta/2) (p^T v) v
-        double pv = 0.0;
-        for (int i = k + 1 + tid; i < n; i += ET) pv += p[i] * v[i];
-        const double K = 0.5 * beta * block_sum(pv, red);
-        for (int i = k + 1 + tid; i < n; i += ET) p[i] -= K * v[i];
-        __syncthreads();
-        // A_sub -= v w^T + w v^T
-        for (int j = k + 1; j < n; ++j) {
-            const double vj = v[j], wj = p[j];
-            for (int i = k + 1 + tid; i < n; i += ET)
-                M[i + (size_t)j * ld] -= v[i] * wj + p[i] * vj;
-        }
-        __syncthreads();
-    }
-    if (tid == 0) {
-        if (n >= 2) {
-            d[n - 2] = M[(n - 2) + (size_t)(n - 2) * ld];
-            e[n - 2] = M[(n - 1) + (size_t)(n - 2) * ld];
-        }
-        d[n - 1] = M[(n - 1) + (size_t)(n - 1) * ld];
-    }
-}
+// eigenvalues by bisection: one thread per requested eigenvalue index, the
+// tridiagonal matrix in shared memory (each count is a chain of n divisions;
+// 13.2 ms at order 441 with its elements read from global memory)
+constexpr int BT = 32;
 
-// eigenvalues by bisection: one thread per requested eigenvalue index
-__global__ void bisect_kernel(const EigEntry* __restrict__ entries, int nwant) {
+__global__ void __launch_bounds__(BT)
+bisect_kernel(const EigEntry* entries, int nwant) {
+    extern __shared__ double esm[];
     const EigEntry en = entries[blockIdx.y];
     const int n = en.n;
-    const int kth = blockIdx.x * blockDim.x + threadIdx.x;
     const int want = nwant > 0 ? min(nwant, n) : n;
-    if (kth >= want) return;
+    if ((int)(blockIdx.x * BT) >= want) return;
+    double *d = esm, *e2 = esm + n;
     double lo = INFINITY, hi = -INFINITY;
-    for (int i = 0; i < n; ++i) {
-        const double r = (i > 0 ? fabs(en.e[i - 1]) : 0.0) + (i + 1 < n ? fabs(en.e[i]) : 0.0);
-        lo = fmin(lo, en.d[i] - r);
-        hi = fmax(hi, en.d[i] + r);
+    for (int i = threadIdx.x; i < n; i += BT) {
+        const double di = en.d[i], ei = i + 1 < n ? en.e[i] : 0.0;
+        const double r = (i > 0 ? fabs(en.e[i - 1]) : 0.0) + fabs(ei);
+        d[i] = di;
+        e2[i] = ei * ei;
+        lo = fmin(lo, di - r);
+        hi = fmax(hi, di + r);
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    __syncwarp();
+    const int kth = blockIdx.x * BT + threadIdx.x;
+    if (kth >= want) return;
     const double pad = 1e-12 * fmax(fabs(lo), fabs(hi)) + 1e-300;
-    en.out[kth] = bisect_kth(en.d, en.e, n, kth, lo - pad, hi + pad);
+    en.out[kth] = bisect_kth(d, e2, n, kth, lo - pad, hi + pad);
 }
 
 }  // namespace
 
 int sym_eigvals_batched(const EigEntry* entries_dev, int count, int nmax, int nwant,
                         cudaStream_t stream) {
-    if (count <= 0) return SCATT_OK;
-    tridiag_kernel<<<count, ET, 0, stream>>>(entries_dev);
+    if (count <= 0 || nmax <= 0) return SCATT_OK;
+    const size_t ts = 3 * (size_t)nmax * sizeof(double), bs = 2 * (size_t)nmax * sizeof(double);
+    if (ts > 200 * 1024) {
+        set_last_error("sym_eigvals_batched: order above 8533");
+        return SCATT_ERR_SIZE;
+    }
+    if (ts > 48 * 1024)
+        SCATT_CUDA_TRY(cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts));
+    if (bs > 48 * 1024)
+        SCATT_CUDA_TRY(cudaFuncSetAttribute(bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bs));
+    tridiag_kernel<<<count * EC, ET, ts, stream>>>(entries_dev);
     const int want = nwant > 0 ? nwant : nmax;
-    dim3 g((want + 127) / 128, count);
-    bisect_kernel<<<g, 128, 0, stream>>>(entries_dev, nwant);
+    bisect_kernel<<<dim3((want + BT - 1) / BT, count), BT, bs, stream>>>(entries_dev, nwant);
     SCATT_CUDA_TRY(cudaGetLastError());
     SCATT_COUNT_LAUNCH(2);
     return SCATT_OK;

@@ -1059,7 +1059,9 @@ int upload_vec(DevBuf<T>& d, const std::vector<T>& h, cudaStream_t s) {
 }
 
 // batched GEMM / GJ helpers for the (non-hot) post stages: entries staged
-// through a small device scratch array
+// through a small device scratch array.  Nothing waits for the device: the
+// entries are copied from pageable memory (staged before the call returns)
+// and the scratch arrays are reused in stream order.
 struct Launcher {
     cudaStream_t s;
     DevBuf<GemmEntry> ge;
@@ -1071,22 +1073,16 @@ struct Launcher {
         for (auto& e : v) { mM = std::max(mM, e.M); mN = std::max(mN, e.N); }
         if (ge.n < v.size()) SCATT_TRY(ge.alloc(v.size()));
         SCATT_CUDA_TRY(cudaMemcpyAsync(ge.p, v.data(), v.size() * sizeof(GemmEntry), cudaMemcpyHostToDevice, s));
-        SCATT_TRY(gemm_batched(ge.p, (int)v.size(), mM, mN, opA, opB, s));
-        return SCATT_CUDA_TRY_RET(cudaStreamSynchronize(s));
+        return gemm_batched(ge.p, (int)v.size(), mM, mN, opA, opB, s);
     }
-    DevBuf<double> gp;   // panel windows for orders above the single-level limit
+    DevBuf<double> gp;   // panel windows of the two-level inverses
     DevBuf<int> gs;
     int gj(const std::vector<GjEntry>& v, bool sym) {
         if (v.empty()) return SCATT_OK;
         int mn = 0;
         for (auto& e : v) mn = std::max(mn, e.n);
         if (je.n < v.size()) SCATT_TRY(je.alloc(v.size()));
-        if (mn <= 1280) {
-            SCATT_CUDA_TRY(cudaMemcpyAsync(je.p, v.data(), v.size() * sizeof(GjEntry), cudaMemcpyHostToDevice, s));
-            SCATT_TRY(gj_inverse_batched(je.p, (int)v.size(), mn, sym, s));
-            return SCATT_CUDA_TRY_RET(cudaStreamSynchronize(s));
-        }
-        // the row-contiguous two-level inverse (cluster panels), 64-column windows, no look-ahead
+        // the two-level inverses by the automatic rule's order, 64-column windows, no look-ahead
         size_t pd = 0, si = 0;
         for (auto& e : v) { pd += 2 * (size_t)e.ld * 64; si += 2 * (size_t)e.n; }
         if (gp.n < pd) SCATT_TRY(gp.alloc(pd));
@@ -1100,8 +1096,8 @@ struct Launcher {
             si += 2 * (size_t)e.n;
         }
         SCATT_CUDA_TRY(cudaMemcpyAsync(je.p, w.data(), w.size() * sizeof(GjEntry), cudaMemcpyHostToDevice, s));
-        SCATT_TRY(gj_inverse_batched3(je.p, (int)w.size(), mn, sym, s, false, -1, 64));
-        return SCATT_CUDA_TRY_RET(cudaStreamSynchronize(s));
+        return mn > 512 ? gj_inverse_batched3(je.p, (int)w.size(), mn, sym, s, false, -1, 64)
+                        : gj_inverse_batched2(je.p, (int)w.size(), mn, sym, s);
     }
     int copy(const std::vector<CopyEntry>& v) {
         if (v.empty()) return SCATT_OK;
@@ -1109,8 +1105,7 @@ struct Launcher {
         SCATT_CUDA_TRY(cudaMemcpyAsync(ce.p, v.data(), v.size() * sizeof(CopyEntry), cudaMemcpyHostToDevice, s));
         k_copy<<<dim3(64, (unsigned)v.size()), TPB, 0, s>>>(ce.p);
         SCATT_COUNT_LAUNCH(1);
-        SCATT_CUDA_TRY(cudaGetLastError());
-        return SCATT_CUDA_TRY_RET(cudaStreamSynchronize(s));
+        return SCATT_CUDA_TRY_RET(cudaGetLastError());
     }
 };
 
@@ -1450,7 +1445,7 @@ size_t post_doubles(const BatchDev& b, int Np, int Nt, int l_cont, int nfit, int
     const size_t np2 = (size_t)Np * Np;
     return 6 * Np + 14 * np2 + (size_t)b.Nf * Np + 2 * (size_t)Nt * Np + 12 * np2 +
            2 * (size_t)(l_cont + 1) * nfit + 8 * (size_t)(l_cont + 1) + 2 * np2 + (size_t)b.Krows * Np +
-           24 * (size_t)Np + 2 * (size_t)n_occ * Np + 8 * (size_t)Np + 2 * np2 + 64;
+           24 * (size_t)Np + 2 * (size_t)n_occ * Np + 8 * (size_t)Np + 2 * np2 + 48 * 32;   // 48 >= the pieces, each rounded up
 }
 // ---------------------------------------------------------------- scan
 struct PostBufs {        // per-energy post-processing buffers
@@ -1681,7 +1676,7 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
     SCATT_TRY(sc.vb.alloc(b));
     {
         const int Np = sc.Np_cap, Nt = sc.Nt_cap;
-        const size_t pd = post_doubles(b, Np, Nt, l_cap, sc.nfit, t.n_occ);
+        const size_t pd = (post_doubles(b, Np, Nt, l_cap, sc.nfit, t.n_occ) + 31) & ~size_t(31);
         SCATT_TRY(sc.parena.alloc(pd * sc.gs));
         SCATT_TRY(sc.pia.alloc((4 * (size_t)Np + 8) * sc.gs));
         sc.P.assign(sc.gs, PostBufs{});
@@ -1690,24 +1685,26 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
             double* p = sc.parena.p + pd * i;
             int* q = sc.pia.p + (4 * (size_t)Np + 8) * i;
             PostBufs& x = sc.P[i];
-            x.tab = p; p += 6 * Np;
-            x.Amat = p; p += np2; x.Bmat = p; p += np2; x.Bw = p; p += np2; x.Binv = p; p += np2;
-            x.Kraw = p; p += np2; x.K = p; p += np2; x.psibc = p; p += np2; x.VP = p; p += np2;
-            x.Bf = p; p += np2; x.rhs = p; p += np2; x.Aaa = p; p += np2; x.Baa = p; p += np2;
-            x.Aw = p; p += np2; x.Ainv = p; p += np2;
-            x.fN = p; p += (size_t)Nf * Np;
-            x.Z0 = p; p += (size_t)Nt * Np; x.Z1 = p; p += (size_t)Nt * Np;
-            x.Q = p; p += 4 * np2; x.Qw = p; p += 4 * np2; x.Qinv = p; p += 4 * np2;
-            x.aatab = p; p += 2 * (size_t)(l_cap + 1) * sc.nfit;
-            x.aaM = p; p += 8 * (size_t)(l_cap + 1);
-            x.aared = p; p += 2 * np2;
-            x.dall = p; p += (size_t)K * Np;
-            x.Dre = p; p += 6 * (size_t)Np; x.Dim = p; p += 6 * (size_t)Np;
-            x.Drre = p; p += 6 * (size_t)Np; x.Drim = p; p += 6 * (size_t)Np;
-            x.ore = p; p += (size_t)t.n_occ * Np; x.oim = p; p += (size_t)t.n_occ * Np;
-            x.ew_d = p; p += 2 * (size_t)Np; x.ew_e = p; p += 2 * (size_t)Np; x.ew_w = p; p += 2 * (size_t)Np;
-            x.eigK = p; p += (size_t)Np; x.eigA = p; p += (size_t)Np;
-            x.Kc = p; p += 2 * np2;
+            // 256-byte aligned pieces, as the inverses need for even orders
+            auto take = [&p](size_t cnt) { double* r = p; p += (cnt + 31) & ~size_t(31); return r; };
+            x.tab = take(6 * Np);
+            x.Amat = take(np2); x.Bmat = take(np2); x.Bw = take(np2); x.Binv = take(np2);
+            x.Kraw = take(np2); x.K = take(np2); x.psibc = take(np2); x.VP = take(np2);
+            x.Bf = take(np2); x.rhs = take(np2); x.Aaa = take(np2); x.Baa = take(np2);
+            x.Aw = take(np2); x.Ainv = take(np2);
+            x.fN = take((size_t)Nf * Np);
+            x.Z0 = take((size_t)Nt * Np); x.Z1 = take((size_t)Nt * Np);
+            x.Q = take(4 * np2); x.Qw = take(4 * np2); x.Qinv = take(4 * np2);
+            x.aatab = take(2 * (size_t)(l_cap + 1) * sc.nfit);
+            x.aaM = take(8 * (size_t)(l_cap + 1));
+            x.aared = take(2 * np2);
+            x.dall = take((size_t)K * Np);
+            x.Dre = take(6 * (size_t)Np); x.Dim = take(6 * (size_t)Np);
+            x.Drre = take(6 * (size_t)Np); x.Drim = take(6 * (size_t)Np);
+            x.ore = take((size_t)t.n_occ * Np); x.oim = take((size_t)t.n_occ * Np);
+            x.ew_d = take(2 * (size_t)Np); x.ew_e = take(2 * (size_t)Np); x.ew_w = take(2 * (size_t)Np);
+            x.eigK = take((size_t)Np); x.eigA = take((size_t)Np);
+            x.Kc = take(2 * np2);
             x.sig = q; q += 2 * Np; x.rid = q; q += 2 * Np; x.st = q; q += 8;
         }
     }
@@ -1990,7 +1987,7 @@ int post_slots(Scan& sc, const std::vector<int>& sel, const std::vector<long>& r
         SCATT_TRY(upload_vec(dnp, np, s));
         SCATT_TRY(upload_vec(dnt, nt, s));
         SCATT_TRY(dnorm.alloc(2 * (size_t)cnt));
-        k_block_norms<<<cnt, TPB, 0, s>>>(dRp.p, dnp.p, dnt.p, dnorm.p);
+        k_block_norms<<<cnt, 1024, 0, s>>>(dRp.p, dnp.p, dnt.p, dnorm.p);
         SCATT_COUNT_LAUNCH(1);
         std::vector<double> norms(2 * cnt);
         SCATT_CUDA_TRY(cudaMemcpyAsync(norms.data(), dnorm.p, norms.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -2205,7 +2202,7 @@ int post_slots(Scan& sc, const std::vector<int>& sel, const std::vector<long>& r
         SCATT_TRY(upload_vec(drp, rp, s));
         SCATT_TRY(upload_vec(drc, rc, s));
         SCATT_TRY(dout.alloc(2 * (size_t)cnt));
-        k_max_pairs<<<cnt, TPB, 0, s>>>(drp.p, drc.p, dout.p);
+        k_max_pairs<<<cnt, 1024, 0, s>>>(drp.p, drc.p, dout.p);
         SCATT_COUNT_LAUNCH(1);
         SCATT_CUDA_TRY(cudaMemcpyAsync(aared.data(), dout.p, 2 * cnt * sizeof(double), cudaMemcpyDeviceToHost, s));
         SCATT_CUDA_TRY(cudaStreamSynchronize(s));
@@ -2245,9 +2242,9 @@ int post_slots(Scan& sc, const std::vector<int>& sel, const std::vector<long>& r
         SCATT_TRY(upload_vec(dnpv, npv, s));
         SCATT_TRY(dsk.alloc(2 * (size_t)cnt));
         SCATT_TRY(dsa.alloc(2 * (size_t)cnt));
-        k_sym_err<<<cnt, TPB, 0, s>>>(dkp.p, dnpv.p, dsk.p);
+        k_sym_err<<<cnt, 1024, 0, s>>>(dkp.p, dnpv.p, dsk.p);
         SCATT_COUNT_LAUNCH(1);
-        k_sym_err<<<cnt, TPB, 0, s>>>(dap.p, dnpv.p, dsa.p);
+        k_sym_err<<<cnt, 1024, 0, s>>>(dap.p, dnpv.p, dsa.p);
         SCATT_COUNT_LAUNCH(1);
         std::vector<double> sk(2 * cnt), sa(2 * cnt);
         SCATT_CUDA_TRY(cudaMemcpyAsync(sk.data(), dsk.p, sk.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
