@@ -289,6 +289,7 @@ __global__ void k_prepare(BatchDev b) {
                       : none;
     const bool inv = n >= b.n_start;
     b.gjR[idx] = GjEntry{d.Ra, d.Rw, rinv, d.sigR, d.ridR, d.stR + 4 * j, inv ? Nt : 0, Nt, Nt, d.PR, d.sgR};
+    if (inv) b.rargs[idx] = RArgs{sinv, d.T, d.F, Dinv_of(b, d, j), rinv_at(b, d, n - 1), Np, Nt, Nf, n < b.n_tr};
     if (inv) b.syR[idx] = sym_entry(d.Ra, d.Rw, d.PR, rinv, b.mag + 4 * (size_t)idx, d.stR + 4 * j, Nt);
     else b.syR[idx].n = 0;
 }
@@ -370,28 +371,25 @@ __global__ void k_stab(BatchDev b, int which) {
         for (int i = threadIdx.x; i < Np; i += blockDim.x) S[i + (size_t)i * Np] += delta;
 }
 
-// Element (i, jc) of R = 12 W^-1 - 10 I - Rinv_prev, W^-1 = [[Sinv, -T], [-T^T, D^-1 + F]].
-struct RElem {
-    const double *sinv, *T, *F, *Dinv, *prev;
-    int Np, Nt, Nf;
-    bool exch;
-    __device__ __forceinline__ RElem(const BatchDev& b, const EnergyDev& d, int n, int j)
-        : sinv(sinv_at(b, d, n, j)), T(d.T), F(d.F), Dinv(Dinv_of(b, d, j)), prev(rinv_at(b, d, n - 1)), Np(d.Np),
-          Nt(d.Nt), Nf(b.Nf), exch(n < b.n_tr) {}
-    __device__ __forceinline__ double operator()(int i, int jc) const {
-        double w;
-        if (i < Np && jc < Np) w = sinv[i + (size_t)jc * Np];
-        else if (i < Np) w = exch ? -T[i + (size_t)(jc - Np) * Np] : 0.0;
-        else if (jc < Np) w = exch ? -T[jc + (size_t)(i - Np) * Np] : 0.0;
-        else {
-            const int fi = i - Np, fj = jc - Np;
-            w = (fi == fj) ? Dinv[fi] : 0.0;
-            if (exch) w += F[fi + (size_t)fj * Nf];
-        }
-        const double u = 12.0 * w - ((i == jc) ? 10.0 : 0.0);
-        return u - prev[i + (size_t)jc * Nt];
-    }
-};
+// Element (i, jc) of R = 12 W^-1 - 10 I - Rinv_prev, W^-1 = [[Sinv, -T],
+// [-T^T, D^-1 + F]]; 0 where !in.  The sources are chosen by selects and read
+// under predicates (no branch keeps one element's loads behind another's).
+__device__ __forceinline__ double r_elem(const RArgs& a, int i, int jc, bool in) {
+    const bool pi = i < a.Np, pj = jc < a.Np;
+    const int fi = i - a.Np, fj = jc - a.Np;
+    const double* src = pi && pj ? a.sinv + i + (size_t)jc * a.Np
+                        : pi     ? a.T + i + (size_t)fj * a.Np
+                        : pj     ? a.T + jc + (size_t)fi * a.Np
+                                 : a.F + fi + (size_t)fj * a.Nf;
+    const bool some = in && ((pi && pj) || a.exch);
+    const bool diag = in && i == jc;
+    double w = some ? *src : 0.0;
+    const double d = diag && !pi ? a.Dinv[fi] : 0.0;
+    const double prev = in ? a.prev[i + (size_t)jc * a.Nt] : 0.0;
+    w = (pi != pj) ? -w : w;
+    const double u = 12.0 * (d + w) - (diag ? 10.0 : 0.0);
+    return u - prev;
+}
 
 // R(n) into Ra, column-major; slots whose step is inside the analytic start skip.
 __global__ void k_assemble_R(BatchDev b, int j) {
@@ -400,12 +398,12 @@ __global__ void k_assemble_R(BatchDev b, int j) {
     const EnergyDev& d = b.ed[e];
     const int n = step_of(b, d, j);
     if (n < b.n_start) return;                 // also n < 0
-    const RElem R(b, d, n, j);
+    const RArgs a = b.rargs[(size_t)j * b.count + e];
     const int Nt = d.Nt;
     const long total = (long)Nt * Nt;
     for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
          idx += (long)gridDim.x * blockDim.x)
-        d.Ra[idx] = R((int)(idx % Nt), (int)(idx / Nt));
+        d.Ra[idx] = r_elem(a, (int)(idx % Nt), (int)(idx / Nt), true);
 }
 
 // The same for one entry of a rescue (sym_rescue_kernel).
@@ -413,28 +411,28 @@ struct RSource {
     BatchDev b;
     int j;
     __device__ __forceinline__ void operator()(int e, const SymEntry& s, int first, int stride) const {
-        const EnergyDev& d = b.ed[e];
-        const RElem R(b, d, step_of(b, d, j), j);
+        const RArgs a = b.rargs[(size_t)j * b.count + e];
         const long total = (long)s.n * s.n;
-        for (long idx = first; idx < total; idx += stride) s.A[idx] = R((int)(idx % s.n), (int)(idx / s.n));
+        for (long idx = first; idx < total; idx += stride)
+            s.A[idx] = r_elem(a, (int)(idx % s.n), (int)(idx / s.n), true);
     }
 };
 
-// R(n) packed for the symmetric sweep; grid (tiles, slots).  Bound by HBM:
-// it reads Sinv, T, F and Rinv(n - 1) once (the lower triangle's half of the
-// symmetric ones) and writes the triangle's tiles.
-__global__ void __launch_bounds__(SYM_THREADS) k_assemble_R_tiles(BatchDev b, int j) {
+// R(n) packed for the symmetric sweep; nt tiles of the largest slot.  Bound
+// by HBM: it reads Sinv, T, F and Rinv(n - 1) once (the lower triangle's half
+// of the symmetric ones) and writes the triangle's tiles.
+__global__ void __launch_bounds__(SYM_THREADS, 3) k_assemble_R_tiles(BatchDev b, int j, int nt) {
     dep_sync();
     extern __shared__ double smem[];
-    const int e = blockIdx.y;
-    const SymEntry s = b.syR[(size_t)j * b.count + e];
+    int ent, t;
+    sym_pack_index(blockIdx.x, b.count, nt, ent, t);
+    const SymEntry s = b.syR[(size_t)j * b.count + ent];
+    const RArgs a = b.rargs[(size_t)j * b.count + ent];
     const int T = sym_tiles_of(s.n);
-    if ((int)blockIdx.x >= T * (T + 1) / 2) return;
-    const EnergyDev& d = b.ed[e];
-    const RElem R(b, d, step_of(b, d, j), j);
+    if (t >= T * (T + 1) / 2) return;
     // the sources are symmetric: taken transposed, consecutive lanes read consecutive rows
-    sym_pack_tile(s, blockIdx.x, *reinterpret_cast<SymDiagShared*>(smem),
-                  [&R](int gi, int gj) { return R(gj, gi); });
+    sym_pack_tile(s, t, *reinterpret_cast<SymDiagShared*>(smem),
+                  [&a](int gi, int gj, bool in) { return r_elem(a, gj, gi, in); });
 }
 
 // Analytic diagonal Rinv for 1 <= n < n_start, 0 at n = 0
@@ -1508,6 +1506,7 @@ struct Scan {
     DevBuf<SymEntry> sy;
     DevBuf<unsigned long long> mag;
     DevBuf<unsigned> barrier;
+    DevBuf<RArgs> rargs;
     VBAt vb;                            // V/B at one step for the post stages
     std::vector<PostBufs> P;            // gs energies
     std::vector<DevBuf<double>> keep;   // stability spectra per l_cont
@@ -1672,6 +1671,8 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
     b.syR = sc.sy.p; b.syS = sc.sy.p + all;
     b.mag = sc.mag.p;
     b.barrier = sc.barrier.p;
+    SCATT_TRY(sc.rargs.alloc(all));
+    b.rargs = sc.rargs.p;
     // ---- post-stage buffers for one group
     SCATT_TRY(sc.vb.alloc(b));
     {
@@ -1849,9 +1850,8 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
             }
             if (rinv[j]) {
                 if (symmetric) {
-                    const int T = sym_tiles_of(sc.Nt_cap);
-                    SCATT_TRY(run(k_assemble_R_tiles, dim3(T * (T + 1) / 2, count), SYM_THREADS, sizeof(SymDiagShared),
-                                  b, j));
+                    const int T = sym_tiles_of(sc.Nt_cap), nt = T * (T + 1) / 2;
+                    SCATT_TRY(run(k_assemble_R_tiles, dim3(count * nt), SYM_THREADS, sizeof(SymDiagShared), b, j, nt));
                 } else {
                     SCATT_TRY(run(k_assemble_R, eg, TPB, 0, b, j));
                 }

@@ -67,6 +67,12 @@ struct EnergyDev {
     double *GA0, *GA1, *wAB, *Mab;
 };
 
+// What R(n) of a slot is made of (k_assemble_R_tiles).
+struct RArgs {
+    const double *sinv, *T, *F, *Dinv, *prev;
+    int Np, Nt, Nf, exch;
+};
+
 // Scan-level constants, static tables and the slot / group arrays.
 struct BatchDev {
     int count;              // slots
@@ -99,6 +105,7 @@ struct BatchDev {
     SymEntry *syS, *syR;
     unsigned long long* mag;
     unsigned* barrier;
+    RArgs* rargs;           // SCHUR_CHUNK x slots
     size_t sw_stride, ps_stride;    // doubles of one Schur slot in Sw and PS
     EnergyDev* ed;
 };

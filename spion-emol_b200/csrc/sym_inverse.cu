@@ -58,15 +58,18 @@ __device__ __forceinline__ void store_out(const SymEntry& e, const double (&acc)
     sym_track_max(m, e.mag + 1);
 }
 
-__global__ void __launch_bounds__(SYM_THREADS)
-sym_pack_kernel(const SymEntry* entries) {
+__global__ void __launch_bounds__(SYM_THREADS, 3)
+sym_pack_kernel(const SymEntry* entries, int count, int nt) {
     dep_sync();
     extern __shared__ double smem[];
-    const SymEntry e = entries[blockIdx.y];
+    int ent, t;
+    sym_pack_index(blockIdx.x, count, nt, ent, t);
+    const SymEntry e = entries[ent];
     const int T = sym_tiles_of(e.n);
-    if ((int)blockIdx.x >= T * (T + 1) / 2) return;
-    sym_pack_tile(e, blockIdx.x, *reinterpret_cast<SymDiagShared*>(smem),
-                  [&e](int gi, int gj) { return e.A[gj + (size_t)gi * e.n]; });
+    if (t >= T * (T + 1) / 2) return;
+    sym_pack_tile(e, t, *reinterpret_cast<SymDiagShared*>(smem), [&e](int gi, int gj, bool in) {
+        return in ? e.A[gj + (size_t)gi * e.n] : 0.0;
+    });
 }
 
 constexpr size_t PANEL_SMEM = 2 * SYM_TILE * sizeof(double);
@@ -283,7 +286,8 @@ int sym_attributes() {
 int sym_pack_batched(const SymEntry* entries_dev, int count, int nmax, cudaStream_t stream) {
     if (count <= 0 || nmax <= 0) return SCATT_OK;
     const int T = sym_tiles_of(nmax);
-    SCATT_CUDA_TRY(launch_dep(sym_pack_kernel, dim3(T * (T + 1) / 2, count), SYM_THREADS, sizeof(SymDiagShared), stream, entries_dev));
+    const int nt = T * (T + 1) / 2;
+    SCATT_CUDA_TRY(launch_dep(sym_pack_kernel, count * nt, SYM_THREADS, sizeof(SymDiagShared), stream, entries_dev, count, nt));
     SCATT_COUNT_LAUNCH(1);
     return SCATT_OK;
 }

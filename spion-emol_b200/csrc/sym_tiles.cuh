@@ -338,9 +338,12 @@ __device__ __forceinline__ void sym_diag_store(const SymEntry& e, int K, const S
     sym_track_max(m, e.mag);
 }
 
-// Packs tile t of entry e from elem(row, column) (row >= 0, column < n; the
-// element of a symmetric matrix, consecutive columns on consecutive lanes)
-// and, for tile 0, inverts the first pivot tile.
+// Packs tile t of entry e from elem(row, column, inside) (the element of a
+// symmetric matrix, consecutive columns on consecutive lanes; anything where
+// !inside, without reading) and, for tile 0, inverts the first pivot tile.
+// elem reads under predicates, not branches, so that a thread's 16 elements
+// are in flight together; one after another they made this pass four times
+// slower than its traffic.
 template <class Elem>
 __device__ __forceinline__ void sym_pack_tile(const SymEntry& e, int t, SymDiagShared& sh, Elem elem) {
     int i = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
@@ -348,26 +351,40 @@ __device__ __forceinline__ void sym_pack_tile(const SymEntry& e, int t, SymDiagS
     while ((size_t)i * (i + 1) / 2 > (size_t)t) --i;
     const int j = t - i * (i + 1) / 2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double* W = e.W + (size_t)t * SYM_TILE;
     const bool first = t == 0;
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        const int gi = i * SYM_NB + warp * 8 + (u >> 1), gj = j * SYM_NB + lane + 32 * (u & 1);
+        v[u] = elem(gi, gj, gi < e.n && gj < e.n);
+    }
     unsigned m = 0;
-#pragma unroll 8
+    double* W = first ? sh.X : e.W + (size_t)t * SYM_TILE;
+#pragma unroll
     for (int u = 0; u < 16; ++u) {
         const int r = warp * 8 + (u >> 1), c = lane + 32 * (u & 1);
         const int gi = i * SYM_NB + r, gj = j * SYM_NB + c;
-        double v = gi == gj ? 1.0 : 0.0;
-        if (gi < e.n && gj < e.n) {
-            v = elem(gi, gj);
-            m = max(m, sym_hi(v));
-        }
-        if (first) sh.X[sym_pos(r, c)] = v;
-        else W[sym_pos(r, c)] = v;
+        const bool in = gi < e.n && gj < e.n;
+        if (in) m = max(m, sym_hi(v[u]));
+        W[sym_pos(r, c)] = in ? v[u] : gi == gj ? 1.0 : 0.0;
     }
     sym_track_hi(m, sym_hi_of_A(e));
     if (first) {
         __syncthreads();
         sym_diag_invert(sh);
         sym_diag_store(e, 0, sh);
+    }
+}
+
+// Entry and tile of CTA bid among count entries of nt tiles: the first tiles,
+// whose pivots are inverted, of all entries come first.
+__device__ __forceinline__ void sym_pack_index(int bid, int count, int nt, int& ent, int& t) {
+    if (bid < count) {
+        ent = bid;
+        t = 0;
+    } else {
+        ent = (bid - count) / (nt - 1);
+        t = 1 + (bid - count) - ent * (nt - 1);
     }
 }
 
