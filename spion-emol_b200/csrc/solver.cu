@@ -2329,7 +2329,7 @@ int post_slots(Scan& sc, const std::vector<int>& sel, const std::vector<long>& r
         auto mat = [&](double* host, const double* dev) -> int {
             if (!host) return SCATT_OK;
             double* h = host + (size_t)ge * Npm * Npm;
-            std::fill(h, h + (size_t)Npm * Npm, 0.0);
+            if (Np < Npm) std::fill(h, h + (size_t)Npm * Npm, 0.0);      // else all of it is copied over
             return cuda_status(cudaMemcpy2D(h, Npm * sizeof(double), dev, Np * sizeof(double), Np * sizeof(double),
                                             Np, cudaMemcpyDeviceToHost), "download");
         };

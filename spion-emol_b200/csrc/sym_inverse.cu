@@ -72,23 +72,26 @@ sym_pack_kernel(const SymEntry* entries, int count, int nt) {
     });
 }
 
-constexpr size_t PANEL_SMEM = 2 * SYM_TILE * sizeof(double);
+constexpr int PANEL_ROWS = 32;
+constexpr size_t PANEL_SMEM = (SYM_TILE + PANEL_ROWS * SYM_NB) * sizeof(double);
 
-// Grid (tile rows, entries).
+// Grid (half tile rows, entries): 32 rows of the pivot column a CTA.  Whole
+// tiles leave a small batch fewer CTAs with a longer chain each, and at 28
+// matrices of order 1046 run as a full wave and a sliver (22 us a launch).
 __global__ void __launch_bounds__(SYM_THREADS, 3)
 sym_panel_kernel(const SymEntry* entries, int K) {
     dep_sync();
     extern __shared__ double smem[];
     const SymEntry e = entries[blockIdx.y];
-    const int T = sym_tiles_of(e.n), i = blockIdx.x;
+    const int T = sym_tiles_of(e.n), i = blockIdx.x >> 1, half = blockIdx.x & 1;
     if (i >= T || K >= T) return;
     const bool last = K == T - 1;
-    double* Ps = smem;
-    double* Ds = smem + SYM_TILE;
+    double* Ds = smem;
+    double* Ps = smem + SYM_TILE;                // 32 x 64: sub-block rows 4 half .. 4 half + 3 of the tile
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wr = warp & 3, wc = warp >> 2;
+    const int wr = warp & 1, wc = warp >> 1;     // 16 rows, 16 columns
     if (i == K) {
-        if (!last) return;
+        if (!last || half) return;
         unsigned long long m = 0;
         for (int u = tid; u < SYM_TILE; u += SYM_THREADS) {
             const int r = u & 63, c = u >> 6;
@@ -101,58 +104,90 @@ sym_panel_kernel(const SymEntry* entries, int K) {
         sym_track_max(m, e.mag + 1);
         return;
     }
+    constexpr int HALF = PANEL_ROWS * SYM_NB;    // doubles
     double* Wt = e.W + (i > K ? sym_tile_index(i, K) : sym_tile_index(K, i)) * SYM_TILE;
-    for (int u = tid; u < SYM_TILE / 2; u += SYM_THREADS) cp16(Ds + 2 * u, e.D + 2 * u);
     if (i > K) {
-        for (int u = tid; u < SYM_TILE / 2; u += SYM_THREADS) cp16(Ps + 2 * u, Wt + 2 * u);
+        for (int u = tid; u < HALF / 2; u += SYM_THREADS) cp16(Ps + 2 * u, Wt + half * HALF + 2 * u);
     } else {
-        for (int u = tid; u < SYM_TILE / 2; u += SYM_THREADS) {
-            const double2 v = reinterpret_cast<const double2*>(Wt)[u];
-            const int sb = u >> 5, row = (u & 31) >> 2, col = (u & 3) * 2;
-            double* d = Ps + ((sb & 7) * 8 + (sb >> 3)) * 64 + row;
+        // rows of the transpose: sub-block columns 4 half .. of tile (K, i)
+#pragma unroll
+        for (int q = 0; q < HALF / 2 / SYM_THREADS; ++q) {
+            const int u = tid + q * SYM_THREADS;                 // sub-block u / 32 of the 8 x 4 read
+            const int sr = u >> 7, sc = (u >> 5) & 3, row = (u & 31) >> 2, col = (u & 3) * 2;
+            const double2 v = *reinterpret_cast<const double2*>(Wt + (sr * 8 + 4 * half + sc) * 64 + row * 8 + col);
+            double* d = Ps + (sc * 8 + sr) * 64 + row;
             d[col * 8] = v.x;
             d[col * 8 + 8] = v.y;
         }
     }
+    for (int u = tid; u < SYM_TILE / 2; u += SYM_THREADS) cp16(Ds + 2 * u, e.D + 2 * u);
     cp_commit();
     cp_wait<0>();
     __syncthreads();
-    double acc[4][4];
+    double acc[2][4];
 #pragma unroll
-    for (int nb = 0; nb < 4; ++nb)
+    for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
         for (int v = 0; v < 4; ++v) acc[nb][v] = 0.0;
-    sym_tile_mma(acc, Ps, Ds, wr, wc, lane, 0, 8);
-    if (last) {
-        // L_i: the inverse's tile (i, K) is -L_i
-        store_out(e, acc, i * SYM_NB, K * SYM_NB, wr, wc, lane);
+#pragma unroll
+    for (int kc = 0; kc < 8; ++kc) {
+        const double2 alo = *reinterpret_cast<const double2*>(Ps + ((2 * wr) * 8 + kc) * 64 + 2 * lane);
+        const double2 ahi = *reinterpret_cast<const double2*>(Ps + ((2 * wr + 1) * 8 + kc) * 64 + 2 * lane);
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+            const double2 b = *reinterpret_cast<const double2*>(Ds + ((2 * wc + nb) * 8 + kc) * 64 + 2 * lane);
+            sym_dmma(acc[nb], alo, ahi, b);
+        }
     }
-    double* Pg = e.P + (size_t)i * SYM_TILE;
-    double* Mg = e.M + (size_t)i * SYM_TILE;
-    for (int u = tid; u < SYM_TILE / 2; u += SYM_THREADS)
+    if (last) {
+        // the inverse's tile (i, K) is -L_i
+        unsigned long long m = 0;
+        const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const int r = i * SYM_NB + half * PANEL_ROWS + wr * 16 + g + ((v >> 1) << 3);
+                const int c = K * SYM_NB + wc * 16 + nb * 8 + 2 * t + (v & 1);
+                if (r >= e.n || c >= e.n) continue;
+                const double x = -acc[nb][v];
+                e.out[r + (size_t)c * e.ldo] = x;
+                e.out[c + (size_t)r * e.ldo] = x;
+                m = max(m, sym_bits(x));
+            }
+        sym_track_max(m, e.mag + 1);
+    }
+    double* Pg = e.P + (size_t)i * SYM_TILE + half * HALF;
+    double* Mg = e.M + (size_t)i * SYM_TILE + half * HALF;
+    for (int u = tid; u < HALF / 2; u += SYM_THREADS)
         reinterpret_cast<double2*>(Pg)[u] = reinterpret_cast<const double2*>(Ps)[u];
 #pragma unroll
-    for (int nb = 0; nb < 4; ++nb)
+    for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int off = ((2 * wr + h) * 8 + 4 * wc + nb) * 64 + 2 * lane;
+            const int off = ((2 * wr + h) * 8 + 2 * wc + nb) * 64 + 2 * lane;
             *reinterpret_cast<double2*>(Mg + off) = make_double2(-acc[nb][2 * h], -acc[nb][2 * h + 1]);
-            if (i > K) *reinterpret_cast<double2*>(Wt + off) = make_double2(acc[nb][2 * h], acc[nb][2 * h + 1]);
+            if (i > K)
+                *reinterpret_cast<double2*>(Wt + half * HALF + off) = make_double2(acc[nb][2 * h], acc[nb][2 * h + 1]);
         }
     if (i < K) {
         __syncthreads();                         // Ps is read by every warp above
         const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-        for (int nb = 0; nb < 4; ++nb)
+        for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
-                // element (row, col) of L_i goes to (col, row) of tile (K, i)
-                double* d = Ps + ((4 * wc + nb) * 8 + 2 * wr + (v >> 1)) * 64;
+                // element (row, col) of L_i goes to (col, row) of tile (K, i): sub-block (col / 8, row / 8) of 8 x 4
+                double* d = Ps + ((2 * wc + nb) * 4 + 2 * wr + (v >> 1)) * 64;
                 d[(2 * t + (v & 1)) * 8 + g] = acc[nb][v];
             }
         __syncthreads();
-        for (int u = tid; u < SYM_TILE / 2; u += SYM_THREADS)
-            reinterpret_cast<double2*>(Wt)[u] = reinterpret_cast<const double2*>(Ps)[u];
+#pragma unroll
+        for (int q = 0; q < HALF / 2 / SYM_THREADS; ++q) {
+            const int u = tid + q * SYM_THREADS;
+            *reinterpret_cast<double2*>(Wt + ((u >> 7) * 8 + 4 * half + ((u >> 5) & 3)) * 64 + (u & 31) * 2) =
+                reinterpret_cast<const double2*>(Ps)[u];
+        }
     }
 }
 
@@ -301,7 +336,7 @@ int sym_sweep_batched(const SymEntry* entries_dev, int count, int nmax, cudaStre
     SCATT_TRY(sym_attributes());
     const int T = sym_tiles_of(nmax), nu = T * (T - 1) / 2;
     for (int K = 0; K < T; ++K) {
-        SCATT_CUDA_TRY(launch_dep(sym_panel_kernel, dim3(T, count), SYM_THREADS, PANEL_SMEM, stream, entries_dev, K));
+        SCATT_CUDA_TRY(launch_dep(sym_panel_kernel, dim3(2 * T, count), SYM_THREADS, PANEL_SMEM, stream, entries_dev, K));
         SCATT_COUNT_LAUNCH(1);
         if (nu > 0) {
             const int ud = K + 1 < T ? K * (K + 1) / 2 + K : -1;

@@ -116,7 +116,8 @@ __device__ __forceinline__ void sym_diag_panel(SymDiagShared& sh, int c, int lan
     bool u0 = (used >> lane) & 1ull, u1 = (used >> (lane + 32)) & 1ull;
     double2* row = reinterpret_cast<double2*>(sh.row);
     double x[8];
-    auto publish = [&](int p) {                  // row p to every lane
+    // row p to every lane, through shared memory (16 shuffles a pivot instead: 43,400 cycles a tile for 40,100)
+    auto publish = [&](int p) {
         if (lane == (p & 31)) {
             if (p < 32) {
 #pragma unroll
@@ -212,7 +213,7 @@ __device__ __forceinline__ void sym_diag_panel(SymDiagShared& sh, int c, int lan
 //
 // Bound by the chain of 64 pivots, each of which stays inside a warp.  A form
 // with the rows spread over the CTA, and one or two barriers a pivot, took
-// 55,000 cycles.  The diagonal is taken where it is at least a quarter of the
+// 55,000 cycles, this one 40,100 (20 us).  The diagonal is taken where it is at least a quarter of the
 // column's largest candidate (nearly always: these matrices are close to
 // diagonal dominance).  Pivoting stays inside the tile: without it (pivots in
 // order) the growth of the intermediate inverses reaches 1e3 to 1e4 and the
