@@ -23,13 +23,6 @@ namespace {
 constexpr int PAD = 4;
 constexpr int THREADS = 128;
 
-__device__ __forceinline__ void dmma_16x8x4(double (&c)[4], double a0, double a1, double b0) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 "
-        "{%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
-        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-        : "d"(a0), "d"(a1), "d"(b0));
-}
 __device__ __forceinline__ void dmma_16x8x8(double (&c)[4], double a0, double a1, double a2, double a3, double b0,
                                             double b1) {
     asm volatile(
@@ -42,110 +35,125 @@ __device__ __forceinline__ void dmma_16x8x8(double (&c)[4], double a0, double a1
 // Thin products (every entry M <= 16: the dipole / overlap row sweeps
 // G(n) = G(n-1) Rinv(n) and their W^-1 terms, K_rows x N_t x N_t).  A
 // 64-row tile would spend three quarters of its DMMAs on zero rows and make
-// these HBM-bound sweeps compute-bound; here a CTA computes 16 x 64 of C
-// with four warps of 16 x 16 and streams op(B) in 32-deep k tiles, staged
-// through registers and double-buffered in shared memory as above.
-constexpr int TBM = 16, TBN = 64, TBK = 32;
+// these HBM-bound sweeps compute-bound; here a CTA computes 16 x 64 of C (16 x
+// 32 where the grid is small) with four warps and streams op(B) through a
+// cp.async ring of 32-deep k stages, 16-byte copies where op(B) = B allows
+// them: a single matrix of order 1046 is a chain of 33 loads, 36 us with one
+// stage in flight, 14 us with three.
+constexpr int TBM = 16, TBK = 32;
+constexpr int T_AKM = TBM + PAD;             // A as [k][m]
+constexpr int T_MK = TBK + PAD;              // A as [m][k], B as [n][k]
 
-template <int OPA, int OPB>
+__device__ __forceinline__ void ring_cp8(double* sdst, const double* gsrc, bool pred) {
+    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" :: "r"(sa), "l"(gsrc), "r"(pred ? 8 : 0));
+}
+__device__ __forceinline__ void ring_cp16(double* sdst, const double* gsrc, bool pred) {
+    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" :: "r"(sa), "l"(gsrc), "r"(pred ? 16 : 0));
+}
+
+template <int OPA, int OPB, int TBN>
+struct ThinLayout {
+    static constexpr int STAGES = TBN == 64 ? 3 : 4;
+    static constexpr int BKN = TBN + PAD;    // B as [k][n]
+    static constexpr int A_ELEMS = OPA == 0 ? TBK * T_AKM : TBM * T_MK;
+    static constexpr int B_ELEMS = OPB == 0 ? TBN * T_MK : TBK * BKN;
+    static constexpr int STAGE = A_ELEMS + B_ELEMS;
+    static constexpr size_t SMEM = STAGES * (size_t)STAGE * sizeof(double);
+};
+
+template <int OPA, int OPB, int TBN>
 __global__ void __launch_bounds__(THREADS)
 gemm_thin_kernel(const GemmEntry* entries) {
     dep_sync();
+    using L = ThinLayout<OPA, OPB, TBN>;
+    constexpr int NB = TBN / 32;                // 8-column blocks of a warp
     const GemmEntry e = entries[blockIdx.z];
     const int n0 = blockIdx.y * TBN;
     if (e.M <= 0 || n0 >= e.N) return;
-    const bool sym = e.sym != 0;
-    if (sym && n0 > 0) return;                  // M = N <= 16: one tile holds the lower triangle
+    const bool sym = e.sym != 0;                // M = N <= 16: one tile holds the lower triangle
 
-    __shared__ double As[2][TBK][TBM + PAD];
-    __shared__ double Bs[2][TBK][TBN + PAD];
-
+    extern __shared__ double tsmem[];
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int wn = warp * 16;
-
-    double acc[2][4];
+    const int nk = (e.K + TBK - 1) / TBK;
+    const bool b16 = OPB == 0 && e.ldb % 2 == 0 && e.K % 2 == 0 && (reinterpret_cast<uintptr_t>(e.B) & 15) == 0;
+    auto issue = [&](int kt, int slot) {
+        if (kt < nk) {
+            double* As = tsmem + slot * L::STAGE;
+            double* Bs = As + L::A_ELEMS;
+            const int k0 = kt * TBK;
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+            for (int u = 0; u < TBM * TBK / THREADS; ++u) {
+                const int idx = tid + u * THREADS;
+                const int m = OPA == 0 ? idx & 15 : idx >> 5, k = OPA == 0 ? idx >> 4 : idx & 31;
+                const bool ok = m < e.M && k0 + k < e.K;
+                const size_t at = OPA == 0 ? m + (size_t)(k0 + k) * e.lda : (k0 + k) + (size_t)m * e.lda;
+                ring_cp8(As + (OPA == 0 ? k * T_AKM + m : m * T_MK + k), e.A + (ok ? at : 0), ok);
+            }
+            if (b16) {
+#pragma unroll
+                for (int u = 0; u < TBN * TBK / 2 / THREADS; ++u) {
+                    const int idx = tid + u * THREADS;
+                    const int n = idx >> 4, k = 2 * (idx & 15);
+                    const bool ok = n0 + n < e.N && k0 + k < e.K;
+                    ring_cp16(Bs + n * T_MK + k, e.B + (ok ? (k0 + k) + (size_t)(n0 + n) * e.ldb : 0), ok);
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < TBN * TBK / THREADS; ++u) {
+                    const int idx = tid + u * THREADS;
+                    const int n = OPB == 0 ? idx >> 5 : idx % TBN, k = OPB == 0 ? idx & 31 : idx / TBN;
+                    const bool ok = n0 + n < e.N && k0 + k < e.K;
+                    const size_t at = OPB == 0 ? (k0 + k) + (size_t)(n0 + n) * e.ldb : (n0 + n) + (size_t)(k0 + k) * e.ldb;
+                    ring_cp8(Bs + (OPB == 0 ? n * T_MK + k : k * L::BKN + n), e.B + (ok ? at : 0), ok);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    double acc[NB][4];
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
 #pragma unroll
         for (int v = 0; v < 4; ++v) acc[j][v] = 0.0;
-
-    double ra[4], rb[16];
-    const int nk = (e.K + TBK - 1) / TBK;
-
-    auto a_at = [&](int i, int& m, int& k) {
-        if (OPA == 0) { m = tid & 15; k = (tid >> 4) + 8 * i; }
-        else          { k = tid & 31; m = (tid >> 5) + 4 * i; }
-    };
-    auto b_at = [&](int i, int& n, int& k) {
-        if (OPB == 0) { k = tid & 31; n = (tid >> 5) + 4 * i; }
-        else          { n = tid & 63; k = (tid >> 6) + 2 * i; }
-    };
-    auto load_tile = [&](int kt) {
-        const int k0 = kt * TBK;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            int m, k;
-            a_at(i, m, k);
-            const int gk = k0 + k;
-            double v = 0.0;
-            if (m < e.M && gk < e.K)
-                v = (OPA == 0) ? e.A[m + (size_t)gk * e.lda] : e.A[gk + (size_t)m * e.lda];
-            ra[i] = v;
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            int n, k;
-            b_at(i, n, k);
-            const int gn = n0 + n, gk = k0 + k;
-            double v = 0.0;
-            if (gn < e.N && gk < e.K)
-                v = (OPB == 0) ? e.B[gk + (size_t)gn * e.ldb] : e.B[gn + (size_t)gk * e.ldb];
-            rb[i] = v;
-        }
-    };
-    auto store_tile = [&](int buf) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            int m, k;
-            a_at(i, m, k);
-            As[buf][k][m] = ra[i];
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            int n, k;
-            b_at(i, n, k);
-            Bs[buf][k][n] = rb[i];
-        }
-    };
-
-    if (nk > 0) {
-        load_tile(0);
-        store_tile(0);
-    }
-    __syncthreads();
-
+    for (int p = 0; p < L::STAGES - 1; ++p) issue(p, p);
+    int slot = 0;
+#pragma unroll 1
     for (int kt = 0; kt < nk; ++kt) {
-        const int buf = kt & 1;
-        if (kt + 1 < nk) load_tile(kt + 1);
+        asm volatile("cp.async.wait_group %0;\n" :: "n"(L::STAGES - 2) : "memory");
+        __syncthreads();                        // stage kt is in, and every warp is done with stage kt - 1
+        issue(kt + L::STAGES - 1, slot == 0 ? L::STAGES - 1 : slot - 1);
+        const double* As = tsmem + slot * L::STAGE;
+        const double* Bs = As + L::A_ELEMS;
 #pragma unroll
-        for (int kk = 0; kk < TBK; kk += 4) {
-            const double a0 = As[buf][kk + t][g];
-            const double a1 = As[buf][kk + t][g + 8];
+        for (int kk = 0; kk < TBK; kk += 8) {
+            double a[4];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) dmma_16x8x4(acc[j], a0, a1, Bs[buf][kk + t][wn + j * 8 + g]);
+            for (int h = 0; h < 2; ++h) {
+                const int k = kk + t + 4 * h;
+                a[2 * h] = OPA == 0 ? As[k * T_AKM + g] : As[g * T_MK + k];
+                a[2 * h + 1] = OPA == 0 ? As[k * T_AKM + g + 8] : As[(g + 8) * T_MK + k];
+            }
+#pragma unroll
+            for (int j = 0; j < NB; ++j) {
+                const int c = (warp * NB + j) * 8 + g, k = kk + t;
+                const double b0 = OPB == 0 ? Bs[c * T_MK + k] : Bs[k * L::BKN + c];
+                const double b1 = OPB == 0 ? Bs[c * T_MK + k + 4] : Bs[(k + 4) * L::BKN + c];
+                dmma_16x8x8(acc[j], a[0], a[1], a[2], a[3], b0, b1);
+            }
         }
-        if (kt + 1 < nk) store_tile(buf ^ 1);
-        __syncthreads();
+        slot = slot == L::STAGES - 1 ? 0 : slot + 1;
     }
-
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int j = 0; j < NB; ++j)
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
             const int row = g + ((v >> 1) << 3);
-            const int col = n0 + wn + j * 8 + 2 * t + (v & 1);
+            const int col = n0 + (warp * NB + j) * 8 + 2 * t + (v & 1);
             if (row < e.M && col < e.N && !(sym && col > row)) {
                 double* c = e.C + row + (size_t)col * e.ldc;
                 double r = e.alpha * acc[j][v];
@@ -158,8 +166,8 @@ gemm_thin_kernel(const GemmEntry* entries) {
 
 // Everything else (some entry M > 16: the Schur update B D^-1 B^T, T = Sinv
 // Bs, F = Bs^T T, the fit rows): 64 x 64 tiles, eight warps of 16 x 32,
-// three CTAs per SM.  k streams through a three-stage cp.async ring of
-// 16-deep stages with one barrier per stage.  Each operand is staged in the
+// three CTAs per SM.  k streams through a three- or eight-stage cp.async
+// ring of 16-deep stages with one barrier per stage.  Each operand is staged in the
 // layout its global storage is contiguous in (A as [k][m] for op N, [m][k]
 // for op T; B as [n][k] for op N, [k][n] for op T), so every copy is a
 // contiguous run: 16-byte copies where the leading dimension, the contiguous
@@ -169,7 +177,7 @@ gemm_thin_kernel(const GemmEntry* entries) {
 // (441 and 605 rows fill 7 and 10 of them to 0.98 and 0.95, but 4 and 5 of
 // 128 to 0.86 and 0.95) and from the symmetric products, whose diagonal tiles
 // waste half.
-constexpr int RB = 64, RK = 16, RTHREADS = 256, RSTAGES = 3;
+constexpr int RB = 64, RK = 16, RTHREADS = 256;
 constexpr int R_KM = RB + PAD;               // [k][m] rows
 constexpr int R_MK = RK + PAD;               // [m][k] rows
 
@@ -178,17 +186,7 @@ struct RingLayout {
     static constexpr int A_ELEMS = OPA == 0 ? RK * R_KM : RB * R_MK;
     static constexpr int B_ELEMS = OPB == 0 ? RB * R_MK : RK * R_KM;
     static constexpr int STAGE = A_ELEMS + B_ELEMS;
-    static constexpr size_t SMEM = RSTAGES * (size_t)STAGE * sizeof(double);
 };
-
-__device__ __forceinline__ void ring_cp8(double* sdst, const double* gsrc, bool pred) {
-    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" :: "r"(sa), "l"(gsrc), "r"(pred ? 8 : 0));
-}
-__device__ __forceinline__ void ring_cp16(double* sdst, const double* gsrc, bool pred) {
-    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" :: "r"(sa), "l"(gsrc), "r"(pred ? 16 : 0));
-}
 
 // One operand's stage: RB rows x (of extent nx) by RK k (of extent nk), stored
 // x-contiguous (XC: X[x + k ld], staged [k][x]) or k-contiguous (staged [x][k]).
@@ -216,7 +214,7 @@ __device__ __forceinline__ void ring_copy(double* sm, const double* X, int ld, i
     }
 }
 
-template <int OPA, int OPB>
+template <int OPA, int OPB, int RSTAGES>
 __global__ void __launch_bounds__(RTHREADS, 3)
 gemm_ring_kernel(const GemmEntry* entries) {
     dep_sync();
@@ -302,20 +300,40 @@ gemm_ring_kernel(const GemmEntry* entries) {
         }
 }
 
-template <int OPA, int OPB>
-int launch_ring(const GemmEntry* entries_dev, int count, int maxM, int maxN, cudaStream_t stream) {
-    using L = RingLayout<OPA, OPB>;
-    static_assert(L::SMEM <= 75 * 1024, "three CTAs per SM");
+template <class Kernel>
+int launch_stages(Kernel kernel, std::atomic<unsigned long long>& done, dim3 grid, int threads, size_t smem,
+                  const GemmEntry* entries_dev, cudaStream_t stream) {
     int dev = 0;
     SCATT_CUDA_TRY(cudaGetDevice(&dev));
-    static std::atomic<unsigned long long> done{0};
     if (dev < 0 || dev >= 64 || !(done.load() & (1ull << dev))) {
-        SCATT_CUDA_TRY(cudaFuncSetAttribute(gemm_ring_kernel<OPA, OPB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)L::SMEM));
+        SCATT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (dev >= 0 && dev < 64) done.fetch_or(1ull << dev);
     }
+    return SCATT_CUDA_TRY_RET(launch_dep(kernel, grid, dim3(threads), smem, stream, entries_dev));
+}
+
+template <int OPA, int OPB>
+int launch_ring(const GemmEntry* entries_dev, int count, int maxM, int maxN, cudaStream_t stream) {
+    constexpr size_t stage = RingLayout<OPA, OPB>::STAGE * sizeof(double);
+    static_assert(3 * stage <= 75 * 1024, "three CTAs per SM");
+    static std::atomic<unsigned long long> done3{0}, done8{0};
     const dim3 grid((maxM + RB - 1) / RB, (maxN + RB - 1) / RB, count);
-    return SCATT_CUDA_TRY_RET(launch_dep(gemm_ring_kernel<OPA, OPB>, grid, RTHREADS, L::SMEM, stream, entries_dev));
+    // A grid that leaves each SM one CTA is a chain of loads: eight stages in
+    // flight instead of three (which let three CTAs share an SM).
+    if ((long)grid.x * grid.y * count <= 148)
+        return launch_stages(gemm_ring_kernel<OPA, OPB, 8>, done8, grid, RTHREADS, 8 * stage, entries_dev, stream);
+    return launch_stages(gemm_ring_kernel<OPA, OPB, 3>, done3, grid, RTHREADS, 3 * stage, entries_dev, stream);
+}
+
+template <int OPA, int OPB>
+int launch_thin(const GemmEntry* entries_dev, int count, int maxN, cudaStream_t stream) {
+    static std::atomic<unsigned long long> done32{0}, done64{0};
+    // 32 columns a CTA spread a grid of at most two waves over more SMs; past that they only read A twice as often
+    if ((long)((maxN + 63) / 64) * count <= 296)
+        return launch_stages(gemm_thin_kernel<OPA, OPB, 32>, done32, dim3(1, (maxN + 31) / 32, count), THREADS,
+                             ThinLayout<OPA, OPB, 32>::SMEM, entries_dev, stream);
+    return launch_stages(gemm_thin_kernel<OPA, OPB, 64>, done64, dim3(1, (maxN + 63) / 64, count), THREADS,
+                         ThinLayout<OPA, OPB, 64>::SMEM, entries_dev, stream);
 }
 
 }  // namespace
@@ -328,13 +346,10 @@ int gemm_batched(const GemmEntry* entries_dev, int count, int maxM, int maxN,
         return SCATT_ERR_ARG;
     }
     if (maxM <= TBM) {
-        cudaError_t le = cudaSuccess;
-        const dim3 tg(1, (maxN + TBN - 1) / TBN, count);
-        if (opA == 0 && opB == 0)      le = launch_dep(gemm_thin_kernel<0, 0>, tg, THREADS, 0, stream, entries_dev);
-        else if (opA == 1 && opB == 0) le = launch_dep(gemm_thin_kernel<1, 0>, tg, THREADS, 0, stream, entries_dev);
-        else if (opA == 0 && opB == 1) le = launch_dep(gemm_thin_kernel<0, 1>, tg, THREADS, 0, stream, entries_dev);
-        else                           le = launch_dep(gemm_thin_kernel<1, 1>, tg, THREADS, 0, stream, entries_dev);
-        SCATT_CUDA_TRY(le);
+        if (opA == 0 && opB == 0)      SCATT_TRY((launch_thin<0, 0>(entries_dev, count, maxN, stream)));
+        else if (opA == 1 && opB == 0) SCATT_TRY((launch_thin<1, 0>(entries_dev, count, maxN, stream)));
+        else if (opA == 0 && opB == 1) SCATT_TRY((launch_thin<0, 1>(entries_dev, count, maxN, stream)));
+        else                           SCATT_TRY((launch_thin<1, 1>(entries_dev, count, maxN, stream)));
         SCATT_COUNT_LAUNCH(1);
         return SCATT_OK;
     }
