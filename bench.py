@@ -23,7 +23,7 @@ e2e        the same steps through the C ABI with host buffers: energies
            submitted from host memory, every output of the finished energies
            read back into pinned host memory, host clock, max over ranks;
 roofline   the dominant kernel group -- the batched R^-1 inversion -- as
-           achieved FP64 TF/s (2 n^3 per matrix, over the sampled inversions)
+           achieved FP64 TF/s (n^3 per matrix, over the sampled inversions)
            against the cuBLAS DGEMM peak measured on this GPU in the same run;
 cpu_baseline  the oracle port timed on a bounded sample of the same workload
            on this host's cores, extrapolated to energies/s.
@@ -66,13 +66,12 @@ DATA = {"h2_like": "synthetic (seeded H2-like inputs of the benchmark shapes)",
         "c8f8_like": "synthetic (seeded C8F8-like inputs of the benchmark shapes)"}
 
 
-# DRAM bytes (read + write) of the trailing updates of one sampled R^-1
-# inversion of the scan, keyed by (config, slots, groups).  From one ncu
-# capture of gj3_trail128_kernel on 32 matrices of order 1046 (452.7 MB for
-# 15 of the 17 column tiles of one 128-column window), scaled to 17 tiles,
-# 128 matrices and the call's 9 windows: the C tiles are read and written
-# once per window, so the traffic grows with the tiles and matrices.
-INVERSE_TRAFFIC: dict = {("h2o_like", 128, 16): 452.7e6 * 17 / 15 * 4 * 9}
+# DRAM bytes (read + write) of the tile updates of one sampled R^-1 inversion
+# of the scan, keyed by (config, slots, groups).  From one ncu capture of
+# sym_update_kernel on 28 matrices of order 1046 (2.64 TB/s over 86.3 us for
+# one pivot tile), scaled to 128 matrices and the call's 16 updates: the
+# triangle's tiles are read and written once per pivot tile.
+INVERSE_TRAFFIC: dict = {("h2o_like", 128, 16): 2.64e12 * 86.3e-6 * 128 / 28 * 16}
 
 
 # Device seconds of one chunk (8 radial steps) with every slot busy, as
@@ -440,8 +439,7 @@ def main():
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": (achieved / peak) if (achieved and peak) else None,
                          "traffic": INVERSE_TRAFFIC.get((a.config, slots, groups)),
-                         "kernel": f"batched R^-1 (Gauss-Jordan, N_t={Nt} in the exchange region, "
-                                   f"{sol.Np} outside; {slots} matrices a call); "
+                         "kernel": f"batched R^-1 (symmetric sweep, N_t={Nt}; {slots} matrices a call); "
                                    "peak = cuBLAS DGEMM 8192^3 measured in this run (FP64 of measured)"},
             "clocks": ck,
             "setup_s": setup_s,

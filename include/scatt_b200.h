@@ -117,7 +117,9 @@ int scatt_bench_inverse(int n, int count, int reps, double* ms_per_call);
 int scatt_bench_gemm(int opA, int opB, int M, int N, int K, int count, int sym, int reps,
                      double* ms_per_call);
 /* Blocking scheme of every dense inverse (the entry points and the solver):
- * 0 = automatic (default): scheme 3 above order 512, scheme 2 below,
+ * 0 = automatic (default): the solver's S(n) and R(n), which are symmetric,
+ *     by the symmetric sweep (scatt_inverse_symmetric_batched); every other
+ *     inverse by scheme 3 above order 512, scheme 2 below,
  * 1 = single-level (rank-16 updates, row pivoting),
  * 2 = two-level column-major (64-column windows, row pivoting),
  * 3 = two-level on the row-contiguous view of the buffer (pivots by columns
@@ -135,9 +137,9 @@ int scatt_set_inverse_blocking(int scheme);
  * with every panel shape that holds order n, on a batch of `count` seeded
  * matrices of order n (reps timed calls each), and keeps the fastest for
  * (current device, n, count).  Under the automatic scheme
- * (scatt_set_inverse_blocking(0)) every later inverse of exactly that order
- * and batch on that device -- the solver's Schur and R^-1 batches included
- * -- uses the kept choice.  Outputs (each may be NULL): the scheme (2 or 3),
+ * (scatt_set_inverse_blocking(0)) every later general inverse of exactly that
+ * order and batch on that device uses the kept choice; the solver's Schur and
+ * R^-1 batches take the symmetric sweep, which has nothing to tune.  Outputs (each may be NULL): the scheme (2 or 3),
  * the panel shape (0..4: 1x8, 2x8, 3x8, 3x12, 5x8 rows per thread x warps;
  * 5: the cluster panel of orders above 1280; 6: the small cluster panel,
  * row-contiguous scheme, orders up to 3072), look-ahead (0/1), the window
@@ -330,8 +332,9 @@ int scatt_scan_close(scatt_scan* scan);
  * on the library stream): out[0] device seconds, out[1] seconds spent in the
  * sampled R^-1 inversions, out[2] number of sampled inversions, out[3] kernel
  * launches issued, out[4] radial-sweep seconds, out[5] post-processing
- * seconds, out[6] floating-point operations of the sampled inversions
- * (2 n^3 per matrix of order n). */
+ * seconds, out[6] floating-point operations of the sampled inversions (n^3
+ * per matrix of order n by the symmetric sweep, 2 n^3 under a forced general
+ * scheme). */
 int scatt_last_stats(scatt_ctx* ctx, double* out7);
 
 /* ------------------------------------------------------ adjoint

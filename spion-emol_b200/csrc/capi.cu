@@ -247,7 +247,7 @@ int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* o
     if (mode) {
         std::vector<unsigned long long> mg(4 * (size_t)count);
         SCATT_CUDA_TRY(cudaMemcpy(mg.data(), dmag.p, mg.size() * sizeof(mg[0]), cudaMemcpyDeviceToHost));
-        for (int b = 0; b < count; ++b) mode[b] = (int)mg[4 * (size_t)b + 3];
+        for (int b = 0; b < count; ++b) mode[b] = (int)(mg[4 * (size_t)b + 3] & 0xffffffffu);
     }
     for (int b = 0; b < count; ++b)
         if (st[2 * b] != DEV_OK) {

@@ -178,7 +178,8 @@ bool inverse_tune_lookup(int n, int count, InverseTune* out);
 void inverse_tune_store(int device, int n, int count, const InverseTune& t);
 
 // Scheme of every dense inverse (entry points and solver): 0 = automatic
-// (row-contiguous two-level above order 512, where its contiguous pivot-row
+// (the solver's symmetric S and R by the symmetric sweep, sym_inverse.cu; else
+// row-contiguous two-level above order 512, where its contiguous pivot-row
 // tiles pay; column-major two-level below), 1 = single-level,
 // 2 = column-major two-level, 3 = row-contiguous two-level, 4 = scheme 3
 // with 128-column windows (where the entries' buffers hold them), 5 / 6 =

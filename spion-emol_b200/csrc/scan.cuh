@@ -58,7 +58,7 @@ struct ScanTables {
 struct SolveStats {
     double device_s = 0.0, rinv_s = 0.0, sweep_s = 0.0, post_s = 0.0;
     double rinv_calls = 0.0;
-    double rinv_flops = 0.0;   // 2 n^3 summed over the matrices of the sampled inversions
+    double rinv_flops = 0.0;   // summed over the matrices of the sampled inversions: n^3 each (symmetric sweep), else 2 n^3
     unsigned long long launches = 0;
 };
 

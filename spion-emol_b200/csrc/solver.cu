@@ -1770,7 +1770,7 @@ int load_group(Scan& sc, int g) {
 
 struct ChunkTiming {
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> rinv;   // sampled R^-1 inversions
-    double flops = 0.0;                                       // 2 n^3 over their matrices
+    double flops = 0.0;                                       // n^3 (general schemes: 2 n^3) over their matrices
 };
 
 // One chunk of SCHUR_CHUNK radial steps for every running group.  With
@@ -1790,6 +1790,10 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
     // S and R are symmetric: the automatic scheme takes the symmetric sweep (half the flops, no
     // column of pivots); the forced schemes keep the general inverse
     const bool symmetric = g_inverse_scheme.load(std::memory_order_relaxed) == 0;
+    // R of one tile stays with the general inverse: the sweep would be one pivot chain, no faster,
+    // and its eight-column panels leave a few times the rounding of the general inverse's sixteen
+    // (an objective's noise at N_t 64: 1.0e-14 against 1.0e-15)
+    const bool sym_r = symmetric && sc.Nt_cap > SYM_NB;
     int live_rinv[SCHUR_CHUNK] = {};
     std::vector<int> live_in(G, 0);
     for (int e = 0; e < count; ++e) live_in[sc.ed[e].grp] += sc.ed[e].live;
@@ -1849,7 +1853,7 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                 SCATT_TRY(run(k_analytic_R_diag, dim3(4, count), TPB, 0, b, j));
             }
             if (rinv[j]) {
-                if (symmetric) {
+                if (sym_r) {
                     const int T = sym_tiles_of(sc.Nt_cap), nt = T * (T + 1) / 2;
                     SCATT_TRY(run(k_assemble_R_tiles, dim3(count * nt), SYM_THREADS, sizeof(SymDiagShared), b, j, nt));
                 } else {
@@ -1862,7 +1866,7 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                     SCATT_TRY(sc.events.get(&a1));
                     SCATT_CUDA_TRY(cudaEventRecord(a0, s));
                 }
-                if (symmetric) {
+                if (sym_r) {
                     SCATT_TRY(sym_sweep_batched(b.syR + at, count, sc.Nt_cap, s));
                     SCATT_TRY(sym_rescue_launch(b.syR + at, count, b.barrier + j, RSource{b, j}, s));
                 } else {
@@ -1875,7 +1879,7 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                     // carried by Rinv(n-1) keeps R from being block-diagonal
                     for (int e = 0; e < count; ++e) {
                         const double n = sc.ed[e].Nt;
-                        tm->flops += 2.0 * n * n * n;
+                        tm->flops += (sym_r ? 1.0 : 2.0) * n * n * n;
                     }
                 }
             }

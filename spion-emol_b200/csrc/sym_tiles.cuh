@@ -27,7 +27,8 @@ struct SymEntry {
     double* D;              // one tile: the inverse of the pivot tile
     double* out;            // n x n, ld ldo: the inverse, both triangles
     // bit patterns of max |D| [0] and max |out| [1]; the high words of max |A|
-    // and of the largest element of the Schur complements [2]; how it was finished [3]
+    // and of the largest element of the Schur complements [2]; how it was
+    // finished, and the high word of max |A| off the diagonal tiles [3]
     unsigned long long* mag;
     int* status;            // DeviceStatus, first failing column
     int n, ldo;
@@ -73,6 +74,8 @@ constexpr int SYM_PANEL_LD = 10;   // doubles of a panel row: 16-byte rows apart
 __device__ __forceinline__ unsigned sym_hi(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
 __device__ __forceinline__ unsigned* sym_hi_of_A(const SymEntry& e) { return reinterpret_cast<unsigned*>(e.mag + 2); }
 __device__ __forceinline__ unsigned* sym_hi_of_schur(const SymEntry& e) { return reinterpret_cast<unsigned*>(e.mag + 2) + 1; }
+__device__ __forceinline__ unsigned* sym_mode(const SymEntry& e) { return reinterpret_cast<unsigned*>(e.mag + 3); }
+__device__ __forceinline__ unsigned* sym_hi_off_diagonal(const SymEntry& e) { return reinterpret_cast<unsigned*>(e.mag + 3) + 1; }
 __device__ __forceinline__ void sym_track_hi(unsigned m, unsigned* dst) {
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) atomicMax(dst, m);
@@ -148,8 +151,7 @@ __device__ __forceinline__ void sym_diag_panel(SymDiagShared& sh, int c, int lan
         const unsigned best = __reduce_max_sync(0xffffffffu, c0 > c1 ? c0 : c1);
         const unsigned hd = (unsigned)__double2hiint(x[k]) & 0x7fffffffu;
         int p = d;
-        // exponents two apart: a factor of four
-        if (((used >> d) & 1ull) || hd + (2u << 20) < (best & 0x7fffffc0u) || hd >= 0x7fe00000u || hd == 0u) {
+        if (((used >> d) & 1ull) || hd < (best & 0x7fffffc0u) || hd >= 0x7fe00000u || hd == 0u) {
             p = 63 - (int)(best & 63u);
             publish(p);
             rp = sym_rcp(x[k]);
@@ -213,9 +215,8 @@ __device__ __forceinline__ void sym_diag_panel(SymDiagShared& sh, int c, int lan
 //
 // Bound by the chain of 64 pivots, each of which stays inside a warp.  A form
 // with the rows spread over the CTA, and one or two barriers a pivot, took
-// 55,000 cycles, this one 40,100 (20 us).  The diagonal is taken where it is at least a quarter of the
-// column's largest candidate (nearly always: these matrices are close to
-// diagonal dominance).  Pivoting stays inside the tile: without it (pivots in
+// 55,000 cycles, this one 40,100 (20 us; 48,000 where every pivot is off the
+// diagonal).  Pivoting is partial, inside the tile: without it (pivots in
 // order) the growth of the intermediate inverses reaches 1e3 to 1e4 and the
 // solver's results lose one to four digits; with it the growth seen is mostly
 // below 2.
@@ -370,6 +371,7 @@ __device__ __forceinline__ void sym_pack_tile(const SymEntry& e, int t, SymDiagS
         W[sym_pos(r, c)] = in ? v[u] : gi == gj ? 1.0 : 0.0;
     }
     sym_track_hi(m, sym_hi_of_A(e));
+    if (i != j) sym_track_hi(m, sym_hi_off_diagonal(e));
     if (first) {
         __syncthreads();
         sym_diag_invert(sh);
