@@ -1490,6 +1490,7 @@ struct Scan {
     int slots = 0, G = 1, gs = 1;
     int l_cap = 0, Np_cap = 0, Nt_cap = 0;
     int chunks_per_sweep = 0;
+    bool general = false;               // S and R by the general inverse under the automatic scheme too
     std::vector<EnergyDev> ed;          // host copy of the slot state (pointers fixed at open)
     std::vector<GroupDev> grp;          // host mirror of the group state
     std::vector<long> job_of;           // submission index held by each slot (-1 empty)
@@ -1789,7 +1790,7 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
     const bool acc = sc.o.keep_window == 0;
     // S and R are symmetric: the automatic scheme takes the symmetric sweep (half the flops, no
     // column of pivots); the forced schemes keep the general inverse
-    const bool symmetric = g_inverse_scheme.load(std::memory_order_relaxed) == 0;
+    const bool symmetric = !sc.general && g_inverse_scheme.load(std::memory_order_relaxed) == 0;
     // R of one tile stays with the general inverse: the sweep would be one pivot chain, no faster,
     // and its eight-column panels leave a few times the rounding of the general inverse's sixteen
     // (an objective's noise at N_t 64: 1.0e-14 against 1.0e-15)
@@ -3009,6 +3010,9 @@ int adj_forward(Context& ctx, const scatt_solve_opts& o_in, int n, const double*
     o.keep_window = 1;                 // the small stages read the window store
     Scan& sc = A.sc;
     SCATT_TRY(scan_open(ctx, o, n, 1, l_cap, sc));
+    // gradients amplify the inverses' rounding (d sigma / d alpha of a small system moved by 1.3e-9 of
+    // itself under the symmetric sweep): they keep the general inverse
+    sc.general = true;
     const BatchDev& b = sc.b;
     const int K = b.Krows, Nf = b.Nf, N = b.N;
     A.segment = segment;
