@@ -242,7 +242,9 @@ __device__ __forceinline__ SymEntry sym_entry(double* A, double* W, double* pane
 // bookkeeping only; one launch for its SCHUR_CHUNK steps, which read nothing
 // that the chunk changes).  Entries of steps outside a slot's chunk, and of
 // stages a step does not take, are empty (M = 0, n = 0): the kernels skip them.
-__global__ void k_prepare(BatchDev b) {
+// An inverse has one of its two entries filled: with `symmetric` the sweep's
+// where the slot's own order is above one tile, else the general inverse's.
+__global__ void k_prepare(BatchDev b, bool symmetric) {
     dep_sync();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx <= SCHUR_CHUNK) b.barrier[idx] = 0;
@@ -272,10 +274,12 @@ __global__ void k_prepare(BatchDev b) {
     const double* Cn = (n < b.n_pts) ? b.Ctab + (size_t)n * K * b.Np_max : nullptr;
     // Bs B^T = B D^-1 B^T and A are symmetric: lower tiles only, mirrored
     b.gmS[idx] = exch ? GemmEntry{Bs, B_of(b, d, j), S, Np, Np, Nf, b.Np_max, b.Np_max, Np, -1.0, 1.0, 1} : none;
+    const bool symS = symmetric && Np > SYM_NB, symR = symmetric && Nt > SYM_NB;
     b.gjS[idx] = GjEntry{S, d.Sw + j * b.sw_stride, sinv, d.sigS + (size_t)j * Np, d.ridS + (size_t)j * Np,
-                         d.stS + 4 * j, Np, Np, Np, d.PS + j * b.ps_stride, d.sgS + (size_t)j * 4 * Np};
-    b.syS[idx] = sym_entry(S, d.Sw + j * b.sw_stride, d.PS + j * b.ps_stride, sinv,
-                           b.mag + 4 * ((size_t)b.count * SCHUR_CHUNK + idx), d.stS + 4 * j, Np);
+                         d.stS + 4 * j, symS ? 0 : Np, Np, Np, d.PS + j * b.ps_stride, d.sgS + (size_t)j * 4 * Np};
+    if (symS) b.syS[idx] = sym_entry(S, d.Sw + j * b.sw_stride, d.PS + j * b.ps_stride, sinv,
+                                     b.mag + 4 * ((size_t)b.count * SCHUR_CHUNK + idx), d.stS + 4 * j, Np);
+    else b.syS[idx].n = 0;
     b.gmT[idx] = exch ? GemmEntry{sinv, Bs, d.T, Np, Nf, Np, Np, b.Np_max, Np, 1.0, 0.0} : none;
     // F = Bs^T Sinv Bs is symmetric: lower tiles only, mirrored
     b.gmF[idx] = exch ? GemmEntry{Bs, d.T, d.F, Nf, Nf, Np, b.Np_max, Np, Nf, 1.0, 0.0, 1} : none;
@@ -288,9 +292,9 @@ __global__ void k_prepare(BatchDev b) {
                                   2 * Np, 1.0, 0.0}
                       : none;
     const bool inv = n >= b.n_start;
-    b.gjR[idx] = GjEntry{d.Ra, d.Rw, rinv, d.sigR, d.ridR, d.stR + 4 * j, inv ? Nt : 0, Nt, Nt, d.PR, d.sgR};
+    b.gjR[idx] = GjEntry{d.Ra, d.Rw, rinv, d.sigR, d.ridR, d.stR + 4 * j, inv && !symR ? Nt : 0, Nt, Nt, d.PR, d.sgR};
     if (inv) b.rargs[idx] = RArgs{sinv, d.T, d.F, Dinv_of(b, d, j), rinv_at(b, d, n - 1), Np, Nt, Nf, n < b.n_tr};
-    if (inv) b.syR[idx] = sym_entry(d.Ra, d.Rw, d.PR, rinv, b.mag + 4 * (size_t)idx, d.stR + 4 * j, Nt);
+    if (inv && symR) b.syR[idx] = sym_entry(d.Ra, d.Rw, d.PR, rinv, b.mag + 4 * (size_t)idx, d.stR + 4 * j, Nt);
     else b.syR[idx].n = 0;
 }
 
@@ -391,13 +395,15 @@ __device__ __forceinline__ double r_elem(const RArgs& a, int i, int jc, bool in)
     return u - prev;
 }
 
-// R(n) into Ra, column-major; slots whose step is inside the analytic start skip.
+// R(n) into Ra, column-major, of the slots whose general inverse takes it (see
+// k_prepare); those whose step is inside the analytic start skip.
 __global__ void k_assemble_R(BatchDev b, int j) {
     dep_sync();
     const int e = blockIdx.y;
     const EnergyDev& d = b.ed[e];
     const int n = step_of(b, d, j);
     if (n < b.n_start) return;                 // also n < 0
+    if (b.gjR[(size_t)j * b.count + e].n == 0) return;
     const RArgs a = b.rargs[(size_t)j * b.count + e];
     const int Nt = d.Nt;
     const long total = (long)Nt * Nt;
@@ -1791,10 +1797,18 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
     // S and R are symmetric: the automatic scheme takes the symmetric sweep (half the flops, no
     // column of pivots); the forced schemes keep the general inverse
     const bool symmetric = !sc.general && g_inverse_scheme.load(std::memory_order_relaxed) == 0;
-    // R of one tile stays with the general inverse: the sweep would be one pivot chain, no faster,
-    // and its eight-column panels leave a few times the rounding of the general inverse's sixteen
-    // (an objective's noise at N_t 64: 1.0e-14 against 1.0e-15)
-    const bool sym_r = symmetric && sc.Nt_cap > SYM_NB;
+    // Orders of one tile stay with the general inverse, slot by slot: the sweep would be one pivot
+    // chain, no faster, and its eight-column panels leave a few times the rounding of the general
+    // inverse's sixteen (an objective's noise at N_t 64: 1.0e-14 against 1.0e-15)
+    bool gen_s = false, sym_s = false, gen_r = false, sym_r = false;     // what the running slots need
+    for (int e = 0; e < count; ++e) {
+        const EnergyDev& d = sc.ed[e];
+        if (!d.live || sc.grp[d.grp].n0 < 0) continue;
+        (symmetric && d.Np > SYM_NB ? sym_s : gen_s) = true;
+        (symmetric && d.Nt > SYM_NB ? sym_r : gen_r) = true;
+    }
+    const int gen_Np = symmetric ? std::min(sc.Np_cap, SYM_NB) : sc.Np_cap;
+    const int gen_Nt = symmetric ? std::min(sc.Nt_cap, SYM_NB) : sc.Nt_cap;
     int live_rinv[SCHUR_CHUNK] = {};
     std::vector<int> live_in(G, 0);
     for (int e = 0; e < count; ++e) live_in[sc.ed[e].grp] += sc.ed[e].live;
@@ -1829,16 +1843,15 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
         SCATT_TRY(run(k_build_B, dim3(cdiv(std::max(b.Np_max * b.n_sigma, b.Nf), 128), G, SCHUR_CHUNK), 128, 0, b));
         SCATT_TRY(run(k_init_S, dim3(64, count, SCHUR_CHUNK), TPB, 0, b));
         if (stab) SCATT_TRY(run(k_stab, dim3(count, SCHUR_CHUNK), TPB, 0, b, 0));
-        SCATT_TRY(run(k_prepare, dim3(cdiv(count * SCHUR_CHUNK, 128)), 128, 0, b));
+        SCATT_TRY(run(k_prepare, dim3(cdiv(count * SCHUR_CHUNK, 128)), 128, 0, b, symmetric));
         if (any_exch) SCATT_TRY(gemm_slots(sc, b.gmS, count * SCHUR_CHUNK, 0, 0, 1));
         if (stab_x) SCATT_TRY(run(k_stab, dim3(count, SCHUR_CHUNK), TPB, 0, b, 1));
-        if (symmetric) {
+        if (sym_s) {
             SCATT_TRY(sym_pack_batched(b.syS, count * SCHUR_CHUNK, sc.Np_cap, s));
             SCATT_TRY(sym_sweep_batched(b.syS, count * SCHUR_CHUNK, sc.Np_cap, s));
             SCATT_TRY(sym_rescue_batched(b.syS, count * SCHUR_CHUNK, b.barrier + SCHUR_CHUNK, s));
-        } else {
-            SCATT_TRY(gj_inverse_selected(b.gjS, count * SCHUR_CHUNK, sc.Np_cap, true, s, true));
         }
+        if (gen_s) SCATT_TRY(gj_inverse_selected(b.gjS, count * SCHUR_CHUNK, gen_Np, true, s, true));
         // ---- the R-ratio recurrence over the chunk's steps
         const dim3 eg(64, count);
         for (int j = 0; j < SCHUR_CHUNK; ++j) {
@@ -1857,9 +1870,8 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                 if (sym_r) {
                     const int T = sym_tiles_of(sc.Nt_cap), nt = T * (T + 1) / 2;
                     SCATT_TRY(run(k_assemble_R_tiles, dim3(count * nt), SYM_THREADS, sizeof(SymDiagShared), b, j, nt));
-                } else {
-                    SCATT_TRY(run(k_assemble_R, eg, TPB, 0, b, j));
                 }
+                if (gen_r) SCATT_TRY(run(k_assemble_R, eg, TPB, 0, b, j));
                 const bool sample = sample_chunk && j == 0;
                 cudaEvent_t a0 = nullptr, a1 = nullptr;
                 if (sample) {
@@ -1870,9 +1882,8 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                 if (sym_r) {
                     SCATT_TRY(sym_sweep_batched(b.syR + at, count, sc.Nt_cap, s));
                     SCATT_TRY(sym_rescue_launch(b.syR + at, count, b.barrier + j, RSource{b, j}, s));
-                } else {
-                    SCATT_TRY(gj_inverse_selected(b.gjR + at, count, sc.Nt_cap, true, s, true));
                 }
+                if (gen_r) SCATT_TRY(gj_inverse_selected(b.gjR + at, count, gen_Nt, true, s, true));
                 if (sample) {
                     SCATT_CUDA_TRY(cudaEventRecord(a1, s));
                     tm->rinv.push_back({a0, a1});
@@ -1880,7 +1891,7 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                     // carried by Rinv(n-1) keeps R from being block-diagonal
                     for (int e = 0; e < count; ++e) {
                         const double n = sc.ed[e].Nt;
-                        tm->flops += (sym_r ? 1.0 : 2.0) * n * n * n;
+                        tm->flops += (symmetric && sc.ed[e].Nt > SYM_NB ? 1.0 : 2.0) * n * n * n;
                     }
                 }
             }
@@ -1898,7 +1909,9 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
         SCATT_TRY(run(k_advance, dim3(1), MAX_GROUPS, 0, b));
         return SCATT_CUDA_TRY_RET(cudaGetLastError());
     };
-    uint64_t key = (stab ? 1u : 0u) | (stab_x ? 2u : 0u) | (any_exch ? 4u : 0u) | ((uint64_t)symmetric << 59);
+    uint64_t key = (stab ? 1u : 0u) | (stab_x ? 2u : 0u) | (any_exch ? 4u : 0u) | ((uint64_t)gen_s << 59) |
+                   ((uint64_t)sym_s << 60) | ((uint64_t)gen_r << 61) | ((uint64_t)sym_r << 62) |
+                   ((uint64_t)symmetric << 63);
     for (int j = 0; j < SCHUR_CHUNK; ++j) {
         const uint64_t bits = (step[j] ? 1u : 0u) | (exch[j] ? 2u : 0u) | (start[j] ? 4u : 0u) |
                               (rinv[j] ? 8u : 0u) | (sweep[j] ? 16u : 0u) | (pts[j] ? 32u : 0u) |
@@ -3010,8 +3023,12 @@ int adj_forward(Context& ctx, const scatt_solve_opts& o_in, int n, const double*
     o.keep_window = 1;                 // the small stages read the window store
     Scan& sc = A.sc;
     SCATT_TRY(scan_open(ctx, o, n, 1, l_cap, sc));
-    // gradients amplify the inverses' rounding (d sigma / d alpha of a small system moved by 1.3e-9 of
-    // itself under the symmetric sweep): they keep the general inverse
+    // The gradients keep the general inverse.  d sigma / d alpha is a sum with much cancellation of
+    // its terms, which shows any change of rounding: from the general inverse to the sweep it moved, over
+    // 40 sets of energies at N_t 196, by 2e-11 of itself in the median and by more than 1e-9 in three (two
+    // blockings of the general inverse differ as much), and gradients are compared with earlier ones.  The
+    // forward's K, A, B and D are therefore those of a solve under the general inverse, bit for bit, and of the
+    // default solve bit for bit up to order 64 and to rounding above.
     sc.general = true;
     const BatchDev& b = sc.b;
     const int K = b.Krows, Nf = b.Nf, N = b.N;
