@@ -222,6 +222,7 @@ int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* o
     SCATT_TRY(dO.alloc(nn * count));
     SCATT_TRY(dP.alloc(ps * count));
     SCATT_TRY(dst.alloc(2 * (size_t)count));
+    SCATT_TRY(dst.zero());
     SCATT_TRY(dmag.alloc(4 * (size_t)count));
     SCATT_TRY(dbar.alloc(1));
     SCATT_TRY(dbar.zero());

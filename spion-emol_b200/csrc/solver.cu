@@ -230,11 +230,12 @@ __device__ __forceinline__ double* gacc_at(const BatchDev& b, const EnergyDev& d
     return (n & 1) ? d.G1 : d.G0;
 }
 
-// Entry of a symmetric inverse of order n (ld n throughout), its magnitudes cleared.
+// Entry of a symmetric inverse of order n (ld n throughout), its magnitudes and status cleared.
 __device__ __forceinline__ SymEntry sym_entry(double* A, double* W, double* panel, double* out,
                                               unsigned long long* mag, int* status, int n) {
     const size_t T = sym_tiles_of(n);
     mag[0] = mag[1] = mag[2] = mag[3] = 0;
+    status[0] = status[1] = 0;
     return SymEntry{A, W, panel, panel + T * SYM_TILE, panel + 2 * T * SYM_TILE, out, mag, status, n, n};
 }
 

@@ -170,6 +170,8 @@ constexpr int SYM_RESCUE_LIST = 256;          // entries looked at in one pass
 
 // `source` fills rows and columns of entry.A from what the caller still has
 // (index, entry, first element, stride); entry.A may also have been kept.
+// The status words come in cleared and are only ever set here, each entry's by
+// one CTA: passes over the list are not ordered between the CTAs.
 template <class Source>
 __global__ void __launch_bounds__(SYM_THREADS, 1)
 sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, Source source) {
@@ -196,11 +198,7 @@ sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, Source 
                 else if (e.n <= SYM_NB) mode = 0;           // one tile: pivoted throughout
                 else if (gr > 1e3) mode = 2;
                 else if (gr > 3.0 || off * d > 2e4) mode = 1;
-                if (blockIdx.x == 0) {
-                    *sym_mode(e) = (unsigned)mode;
-                    e.status[0] = 0;
-                    e.status[1] = 0;
-                }
+                if (blockIdx.x == 0) *sym_mode(e) = (unsigned)mode;
             }
             s_mode[k] = mode;
             any |= mode;

@@ -30,7 +30,7 @@ struct SymEntry {
     // and of the largest element of the Schur complements [2]; how it was
     // finished, and the high word of max |A| off the diagonal tiles [3]
     unsigned long long* mag;
-    int* status;            // DeviceStatus, first failing column
+    int* status;            // DeviceStatus, first failing column; zero before the sweep
     int n, ldo;
 };
 
@@ -394,7 +394,7 @@ __device__ __forceinline__ void sym_pack_index(int bid, int count, int nt, int& 
 // Sweeps a packed batch (pivot tile 0 already inverted) to the inverses, all
 // entries of order <= nmax; entries of order 0 are skipped.
 int sym_sweep_batched(const SymEntry* entries_dev, int count, int nmax, cudaStream_t stream);
-// Packs full symmetric matrices (entry.A) for sym_sweep_batched; mag must be zero.
+// Packs full symmetric matrices (entry.A) for sym_sweep_batched; mag and status must be zero.
 int sym_pack_batched(const SymEntry* entries_dev, int count, int nmax, cudaStream_t stream);
 
 }  // namespace scatt

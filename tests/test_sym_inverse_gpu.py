@@ -71,3 +71,32 @@ def test_singular_and_nonfinite_are_reported():
     assert st[0, 0] == 1 and st[1, 0] == 0 and st[2, 0] == 2
     ref = np.linalg.inv(A[1])
     assert np.max(np.abs(X[1] - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+def test_statuses_of_a_long_batch():
+    """More matrices than one pass of the rescue looks at (256): slow pivoted
+    eliminations in the first pass, failing matrices in both."""
+    n, count = 200, 600
+    A = np.repeat(symmetric(np.random.default_rng(3), 1, n), count, axis=0)
+    rescued = [0, 148, 255, 300]                    # leading block zero, as in the test above: regular
+    for b in rescued:
+        A[b, :64, :64] = 0.0
+        A[b, :64, 64:128] = A[b, 64:128, :64] = np.eye(64)
+        A[b, :64, 128:] = A[b, 128:, :64] = 0.0
+    singular, bad = [3, 149, 256, 297, 440, 599], [5, 254, 258, 400, 513]
+    for b in singular:
+        A[b, 70, :] = A[b, :, 70] = 0.0
+    for b in bad:
+        A[b, 5, 5] = np.nan
+    want = np.zeros(count, dtype=int)
+    want[singular], want[bad] = 1, 2
+    X, st, mode = _lib.inverse_symmetric_batched(A)
+    assert np.array_equal(st[:, 0], want)
+    assert np.all(mode[rescued + singular + bad] == 3) and np.count_nonzero(mode) == len(rescued + singular + bad)
+    good = np.linalg.inv(A[1])
+    for b in range(count):
+        if want[b] == 0 and b not in rescued:
+            assert np.max(np.abs(X[b] - good)) <= 1e-12 * np.max(np.abs(good))
+    for b in rescued:
+        ref = np.linalg.inv(A[b])
+        assert np.max(np.abs(X[b] - ref)) <= 1e-13 * max(10.0, np.linalg.cond(A[b])) * np.max(np.abs(ref))
