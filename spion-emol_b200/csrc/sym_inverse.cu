@@ -72,12 +72,37 @@ sym_pack_kernel(const SymEntry* entries, int count, int nt) {
     });
 }
 
+// acc (16 x 16 of a 32 x 64 product, warp (wr, wc)) += A B^T over the shared half tile As and tile Bs.
+__device__ __forceinline__ void sym_half_mma(double (&acc)[2][4], const double* As, const double* Bs, int wr, int wc,
+                                             int lane) {
+#pragma unroll
+    for (int kc = 0; kc < 8; ++kc) {
+        const double2 alo = *reinterpret_cast<const double2*>(As + ((2 * wr) * 8 + kc) * 64 + 2 * lane);
+        const double2 ahi = *reinterpret_cast<const double2*>(As + ((2 * wr + 1) * 8 + kc) * 64 + 2 * lane);
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+            const double2 b = *reinterpret_cast<const double2*>(Bs + ((2 * wc + nb) * 8 + kc) * 64 + 2 * lane);
+            sym_dmma(acc[nb], alo, ahi, b);
+        }
+    }
+}
+
 constexpr int PANEL_ROWS = 32;
 constexpr size_t PANEL_SMEM = (SYM_TILE + PANEL_ROWS * SYM_NB) * sizeof(double);
 
 // Grid (half tile rows, entries): 32 rows of the pivot column a CTA.  Whole
 // tiles leave a small batch fewer CTAs with a longer chain each, and at 28
 // matrices of order 1046 run as a full wave and a sliver (22 us a launch).
+//
+// L = P D takes over D's error, kappa(A_KK) eps, and the update L P^T multiplies
+// it by P again, where the Schur complement may cancel to a small part of
+// P D P^T: a matrix with one dominant direction (c / n v v^T beside a part of
+// norm 1, c = 1e5, order 196) lost four digits, 1.6e-9 against the pivoted
+// elimination's 5.5e-13.  Where the tile's skew tells of it, one step by the
+// tile itself, L += (P - L A_KK) D, leaves the row residual at rounding
+// whatever kappa: 8.6e-13.  Only there: two products more of 64 x 64 a CTA.
+// Telling costs the inverse 2 % (order 1046: 28 matrices 1.763 -> 1.796 ms,
+// one 0.589 -> 0.601), as the pivot tile is kept and read again.
 __global__ void __launch_bounds__(SYM_THREADS, 3)
 sym_panel_kernel(const SymEntry* entries, int K) {
     dep_sync();
@@ -129,15 +154,37 @@ sym_panel_kernel(const SymEntry* entries, int K) {
     for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
         for (int v = 0; v < 4; ++v) acc[nb][v] = 0.0;
+    sym_half_mma(acc, Ps, Ds, wr, wc, lane);
+    double* Pg = e.P + (size_t)i * SYM_TILE + half * HALF;
+    double* Mg = e.M + (size_t)i * SYM_TILE + half * HALF;
+    for (int u = tid; u < HALF / 2; u += SYM_THREADS)
+        reinterpret_cast<double2*>(Pg)[u] = reinterpret_cast<const double2*>(Ps)[u];
+    if (*sym_skew(e) > SYM_SKEW_MAX) {           // the same for the CTA
+        double res[2][4];                        // P - L A_KK
+        const double2 *A2 = reinterpret_cast<const double2*>(sym_tile_of_D(e)), *D2 = reinterpret_cast<const double2*>(e.D);
+        __syncthreads();                         // Ps and Ds are read by every warp above
 #pragma unroll
-    for (int kc = 0; kc < 8; ++kc) {
-        const double2 alo = *reinterpret_cast<const double2*>(Ps + ((2 * wr) * 8 + kc) * 64 + 2 * lane);
-        const double2 ahi = *reinterpret_cast<const double2*>(Ps + ((2 * wr + 1) * 8 + kc) * 64 + 2 * lane);
+        for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
-        for (int nb = 0; nb < 2; ++nb) {
-            const double2 b = *reinterpret_cast<const double2*>(Ds + ((2 * wc + nb) * 8 + kc) * 64 + 2 * lane);
-            sym_dmma(acc[nb], alo, ahi, b);
-        }
+            for (int h = 0; h < 2; ++h) {
+                double2* p = reinterpret_cast<double2*>(Ps + ((2 * wr + h) * 8 + 2 * wc + nb) * 64 + 2 * lane);
+                res[nb][2 * h] = p->x;
+                res[nb][2 * h + 1] = p->y;
+                *p = make_double2(-acc[nb][2 * h], -acc[nb][2 * h + 1]);
+            }
+        for (int u = tid; u < SYM_TILE / 2; u += SYM_THREADS) reinterpret_cast<double2*>(Ds)[u] = A2[u];
+        __syncthreads();
+        sym_half_mma(res, Ps, Ds, wr, wc, lane);
+        __syncthreads();
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<double2*>(Ps + ((2 * wr + h) * 8 + 2 * wc + nb) * 64 + 2 * lane) =
+                    make_double2(res[nb][2 * h], res[nb][2 * h + 1]);
+        for (int u = tid; u < SYM_TILE / 2; u += SYM_THREADS) reinterpret_cast<double2*>(Ds)[u] = D2[u];
+        __syncthreads();
+        sym_half_mma(acc, Ps, Ds, wr, wc, lane);
     }
     if (last) {
         // the inverse's tile (i, K) is -L_i
@@ -157,10 +204,6 @@ sym_panel_kernel(const SymEntry* entries, int K) {
             }
         sym_track_max(m, e.mag + 1);
     }
-    double* Pg = e.P + (size_t)i * SYM_TILE + half * HALF;
-    double* Mg = e.M + (size_t)i * SYM_TILE + half * HALF;
-    for (int u = tid; u < HALF / 2; u += SYM_THREADS)
-        reinterpret_cast<double2*>(Pg)[u] = reinterpret_cast<const double2*>(Ps)[u];
 #pragma unroll
     for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
@@ -293,7 +336,7 @@ sym_update_kernel(const SymEntry* entries, int count, int K, int nu, int ud) {
                 *reinterpret_cast<double2*>(sh.X + ((2 * wr + h) * 8 + 4 * wc + nb) * 64 + 2 * lane) =
                     make_double2(acc[nb][2 * h], acc[nb][2 * h + 1]);
         __syncthreads();
-        sym_diag_invert(sh);
+        sym_diag_invert(sh, sym_tile_of_D(e));
         sym_diag_store(e, K + 1, sh);
         return;
     }

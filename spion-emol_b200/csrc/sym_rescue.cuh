@@ -3,20 +3,17 @@
 // once when no entry needs it.
 //
 // A sweep's error grows with g, the larger of max|D| / max|A^-1| and of the
-// Schur complements' largest element over A's, and with max|D| times A's
-// largest element off the diagonal tiles, where A holds one dominant direction
-// that every tile has a part of.  The inverse takes a Newton step
+// Schur complements' largest element over A's.  The inverse takes a Newton step
 // X <- X (2 I - A X), two products over the whole grid for that entry alone,
-// which squares the relative error, where g > 3 or that product is above 2e4
-// (about 1 in 50 matrices of a radial sweep at a step of 0.05 bohr, and fewer
-// the finer the grid), and a second one above g = 1e3.  Not elsewhere: the
-// step leaves rounding of kappa eps, which a sweep of a graded matrix (large
-// diagonal elements near the origin) stays ten times below.
+// which squares the relative error, where g > 3 (rare in a radial sweep, and
+// rarer the finer the grid), and a second one above g = 1e3.  Not elsewhere: the step leaves rounding of
+// kappa eps, which a sweep of a graded matrix (large diagonal elements near
+// the origin) stays ten times below.  What a badly conditioned pivot tile does
+// without growth is met in the sweep itself (SYM_SKEW_MAX).
 // Measured on the matrices of one sweep (order 1046, kappa = max|A| max|X|),
 // relative errors:
 //              g       kappa   sweep    Newton   LU       Gauss-Jordan, pivoted
 //              1200    21      3.9e-11  7.7e-16  8.4e-16  1.1e-14
-//              0.94    2.1e6   3.1e-9   8.2e-13  1.9e-12  2.7e-13
 //              15      1.4e3   7.7e-13  7.0e-15  3.9e-13  7.4e-13
 //   median     1       20      7e-16             6e-16
 // Past g = 1e6, and on zero and non-finite pivots, to report them, the entry
@@ -192,12 +189,11 @@ sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, Source 
                 const double d = __longlong_as_double((long long)e.mag[0]);
                 const double x = __longlong_as_double((long long)e.mag[1]);
                 const double a = __hiloint2double((int)*sym_hi_of_A(e), 0), s = __hiloint2double((int)*sym_hi_of_schur(e), 0);
-                const double off = __hiloint2double((int)*sym_hi_off_diagonal(e), 0);
                 const double gr = fmax(d / x, s / a);
                 if (!isfinite(d) || !isfinite(x) || !isfinite(a) || !(x > 0.0) || !(gr <= 1e6)) mode = 3;
                 else if (e.n <= SYM_NB) mode = 0;           // one tile: pivoted throughout
                 else if (gr > 1e3) mode = 2;
-                else if (gr > 3.0 || off * d > 2e4) mode = 1;
+                else if (gr > 3.0) mode = 1;
                 if (blockIdx.x == 0) *sym_mode(e) = (unsigned)mode;
             }
             s_mode[k] = mode;

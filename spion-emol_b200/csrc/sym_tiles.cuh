@@ -24,11 +24,11 @@ struct SymEntry {
     double* A;              // n x n, ld n (both triangles): rebuilt or kept for the rescue, then its scratch
     double* W;              // T (T + 1) / 2 tiles, and two n x n matrices for the rescue
     double *P, *M;          // T tiles each: the pivot column block and its negated product with D
-    double* D;              // one tile: the inverse of the pivot tile
+    double* D;              // the inverse of the pivot tile, the pivot tile itself, and sym_skew of the two
     double* out;            // n x n, ld ldo: the inverse, both triangles
     // bit patterns of max |D| [0] and max |out| [1]; the high words of max |A|
     // and of the largest element of the Schur complements [2]; how it was
-    // finished, and the high word of max |A| off the diagonal tiles [3]
+    // finished [3]
     unsigned long long* mag;
     int* status;            // DeviceStatus, first failing column; zero before the sweep
     int n, ldo;
@@ -36,12 +36,12 @@ struct SymEntry {
 
 __host__ __device__ inline int sym_tiles_of(int n) { return (n + SYM_NB - 1) / SYM_NB; }
 __host__ __device__ inline size_t sym_tile_index(int i, int j) { return (size_t)i * (i + 1) / 2 + j; }
-// Doubles that W needs for order n, and those of P, M and D together.
+// Doubles that W needs for order n, and those of P, M and D together (D: two tiles and a word).
 inline size_t sym_work_doubles(int n) {
     const size_t T = sym_tiles_of(n), w = T * (T + 1) / 2 * SYM_TILE, full = 2 * (size_t)n * n;
     return w > full ? w : full;
 }
-inline size_t sym_panel_doubles(int n) { return (2 * (size_t)sym_tiles_of(n) + 1) * SYM_TILE; }
+inline size_t sym_panel_doubles(int n) { return (2 * (size_t)sym_tiles_of(n) + 2) * SYM_TILE + 32; }
 
 __device__ __forceinline__ int sym_pos(int r, int c) {
     return (((r >> 3) << 3) + (c >> 3)) * 64 + ((r & 7) << 3) + (c & 7);
@@ -75,7 +75,6 @@ __device__ __forceinline__ unsigned sym_hi(double v) { return (unsigned)__double
 __device__ __forceinline__ unsigned* sym_hi_of_A(const SymEntry& e) { return reinterpret_cast<unsigned*>(e.mag + 2); }
 __device__ __forceinline__ unsigned* sym_hi_of_schur(const SymEntry& e) { return reinterpret_cast<unsigned*>(e.mag + 2) + 1; }
 __device__ __forceinline__ unsigned* sym_mode(const SymEntry& e) { return reinterpret_cast<unsigned*>(e.mag + 3); }
-__device__ __forceinline__ unsigned* sym_hi_off_diagonal(const SymEntry& e) { return reinterpret_cast<unsigned*>(e.mag + 3) + 1; }
 __device__ __forceinline__ void sym_track_hi(unsigned m, unsigned* dst) {
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) atomicMax(dst, m);
@@ -89,7 +88,22 @@ struct SymDiagShared {
     unsigned long long took[2];                  // those of the last panel, by parity
     int prow[SYM_NB];                            // row of each step's pivot
     int krow[SYM_NB];                            // step at which each row was the pivot
+    double skew[SYM_THREADS / 32];               // each warp's part of sym_skew
 };
+
+// Pivot tiles whose largest column sum of |A_ij D_ij| (A the tile, D its
+// inverse) is above this have their rows L = P D refined (sym_panel_kernel).
+// The sum is 1 for a diagonal or a well-conditioned dominant tile, does not
+// change when rows and columns are scaled alike (a tile graded by its
+// centrifugal terms has a condition number of 1e3 and a sum below 1.4), and
+// grows with the rounding that D brings into L P^T.  Up to 4, sweeps without
+// the refinement stayed within 1.5 of the general inverse's error over the
+// matrices of radial sweeps (orders 162 and 196, 20 and 50 bohr); above, they
+// did not always.  At 1.4 bohr no tile is above 2, at 20 bohr and order 1046
+// one in 50.
+constexpr double SYM_SKEW_MAX = 2.0;
+__device__ __forceinline__ double* sym_tile_of_D(const SymEntry& e) { return e.D + SYM_TILE; }
+__device__ __forceinline__ double* sym_skew(const SymEntry& e) { return e.D + 2 * SYM_TILE; }
 
 __device__ __forceinline__ void sym_dmma(double (&c)[4], const double2& alo, const double2& ahi, const double2& b);
 
@@ -211,7 +225,8 @@ __device__ __forceinline__ void sym_diag_panel(SymDiagShared& sh, int c, int lan
 // applies it to its own block by DMMAs and goes on to the next panel, and the
 // other warps apply it meanwhile.  Rows are not moved: row p_k of step k ends
 // as row k of the inverse, whose column p_j sits in column j.  The result is
-// symmetrised and left in sh.X.
+// symmetrised and left in sh.X; the tile itself goes to `tile`, and sh.skew
+// gets the column sums of SYM_SKEW_MAX.
 //
 // Bound by the chain of 64 pivots, each of which stays inside a warp.  A form
 // with the rows spread over the CTA, and one or two barriers a pivot, took
@@ -220,7 +235,7 @@ __device__ __forceinline__ void sym_diag_panel(SymDiagShared& sh, int c, int lan
 // order) the growth of the intermediate inverses reaches 1e3 to 1e4 and the
 // solver's results lose one to four digits; with it the growth seen is mostly
 // below 2.
-__device__ __forceinline__ void sym_diag_invert(SymDiagShared& sh) {
+__device__ __forceinline__ void sym_diag_invert(SymDiagShared& sh, double* tile) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     // a lane's element (r, c) of the warp's u-th 8 x 4 patch, and its mirror image: at most four-way conflicts
@@ -237,6 +252,12 @@ __device__ __forceinline__ void sym_diag_invert(SymDiagShared& sh) {
     }
     if (tid == 0) sh.used = 0;
     __syncthreads();
+    // every warp its own column block, which no other changes before the first panel is applied
+#pragma unroll
+    for (int R = 0; R < 8; ++R) {
+        const int off = (R * 8 + warp) * 64 + 2 * lane;
+        *reinterpret_cast<double2*>(tile + off) = *reinterpret_cast<const double2*>(sh.X + off);
+    }
     // block <- (block with the panel's pivot rows zeroed) + panel * (pivot rows of the block)
     auto apply = [&](int c) {
         const double* pan = sh.panel[c & 1];
@@ -277,15 +298,33 @@ __device__ __forceinline__ void sym_diag_invert(SymDiagShared& sh) {
         __syncthreads();
         if (warp != c && warp != c + 1) apply(c);
     }
-    __syncthreads();
-    // inverse(r, c) = X(p_r, step of c), symmetrised
-    double v[16];
+    double v[16];                                // the tile's elements, then the inverse's
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
         int r, c;
         patch(u, r, c);
-        v[u] = 0.5 * (sh.X[sym_pos(sh.prow[r], sh.krow[c])] + sh.X[sym_pos(sh.prow[c], sh.krow[r])]);
+        v[u] = __ldcg(tile + sym_pos(r, c));
     }
+    __syncthreads();
+    // inverse(r, c) = X(p_r, step of c), symmetrised; a lane's patches lie in two columns, by parity of u
+    double sum[2] = {0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+        int r, c;
+        patch(u, r, c);
+        const double x = 0.5 * (sh.X[sym_pos(sh.prow[r], sh.krow[c])] + sh.X[sym_pos(sh.prow[c], sh.krow[r])]);
+        sum[u & 1] += fabs(x * v[u]);
+        v[u] = x;
+    }
+#pragma unroll
+    for (int o = 16; o >= 4; o >>= 1) {
+        sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], o);
+        sum[1] += __shfl_xor_sync(0xffffffffu, sum[1], o);
+    }
+    sum[0] = fmax(sum[0], sum[1]);
+#pragma unroll
+    for (int o = 2; o >= 1; o >>= 1) sum[0] = fmax(sum[0], __shfl_xor_sync(0xffffffffu, sum[0], o));
+    if (lane == 0) sh.skew[warp] = sum[0];
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
@@ -338,6 +377,11 @@ __device__ __forceinline__ void sym_diag_store(const SymEntry& e, int K, const S
         if (row < e.n && col + 1 < e.n) m = max(m, sym_bits(v.y));
     }
     sym_track_max(m, e.mag);
+    if (threadIdx.x == 0) {
+        double s = sh.skew[0];
+        for (int w = 1; w < SYM_THREADS / 32; ++w) s = fmax(s, sh.skew[w]);
+        *sym_skew(e) = s;
+    }
 }
 
 // Packs tile t of entry e from elem(row, column, inside) (the element of a
@@ -371,10 +415,9 @@ __device__ __forceinline__ void sym_pack_tile(const SymEntry& e, int t, SymDiagS
         W[sym_pos(r, c)] = in ? v[u] : gi == gj ? 1.0 : 0.0;
     }
     sym_track_hi(m, sym_hi_of_A(e));
-    if (i != j) sym_track_hi(m, sym_hi_off_diagonal(e));
     if (first) {
         __syncthreads();
-        sym_diag_invert(sh);
+        sym_diag_invert(sh, sym_tile_of_D(e));
         sym_diag_store(e, 0, sh);
     }
 }

@@ -100,3 +100,39 @@ def test_statuses_of_a_long_batch():
     for b in rescued:
         ref = np.linalg.inv(A[b])
         assert np.max(np.abs(X[b] - ref)) <= 1e-13 * max(10.0, np.linalg.cond(A[b])) * np.max(np.abs(ref))
+
+
+def _solutions(A, X, b):
+    """A^-1 b to 64-bit rounding: a few refinements with extended residuals."""
+    Al, x = A.astype(np.longdouble), (X @ b).astype(np.longdouble)
+    for _ in range(5):
+        x = x + X @ (b - Al @ x).astype(np.float64)
+    return x.astype(np.float64)
+
+
+@pytest.mark.parametrize("n", [130, 196, 452, 1046])
+@pytest.mark.parametrize("kind", ["one", "four", "graded"])
+def test_dominant_directions(n, kind):
+    """A part of norm c, which every tile has a share of, beside the family
+    above: the pivot tiles' condition grows with c without any growth of the
+    intermediate inverses.  The error is held to ten times the general
+    inverse's (whose pivots run down the whole matrix); a sweep that takes D
+    at its word loses log10(c) digits more, 1e3 times that bound at c = 1e6."""
+    cs = [1.0, 1e1, 1e2, 1e3, 1e4, 1e5, 1e6]
+    rng = np.random.default_rng(n)
+    B = symmetric(rng, 1, n)[0]
+    v = rng.standard_normal((n, 4 if kind == "four" else 1))
+    if kind == "graded":
+        v *= 10.0 ** (-2.0 * np.arange(n) / n)[:, None]
+    sign = np.array([1.0, -1.0, 1.0, -1.0])[: v.shape[1]]
+    A = np.stack([B + c / n * (v * sign) @ v.T for c in cs])
+    A = 0.5 * (A + np.swapaxes(A, 1, 2))
+    X, st, _ = _lib.inverse_symmetric_batched(A)
+    G, _ = _lib.inverse_batched(A, symmetrize=True)
+    assert np.all(st == 0)
+    b = rng.standard_normal((n, 4))
+    for a, x, g, c in zip(A, X, G, cs):
+        t = _solutions(a, np.linalg.inv(a), b)
+        err = lambda y: np.linalg.norm(y @ b - t) / np.linalg.norm(t)  # noqa: E731
+        # the floor: rounding of the products X b themselves
+        assert err(x) <= 10.0 * err(g) + 1e-15, (c, err(x), err(g))
