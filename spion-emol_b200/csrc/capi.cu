@@ -215,7 +215,8 @@ int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* o
     const size_t ws = (sym_work_doubles(n) + al) & ~al, ps = sym_panel_doubles(n);
     DevBuf<double> dA, dW, dO, dP;
     DevBuf<int> dst;
-    DevBuf<unsigned long long> dmag;
+    DevBuf<unsigned> dstat;
+    const size_t words = sym_stat_words(n);
     DevBuf<unsigned> dbar;
     SCATT_TRY(dA.alloc(nn * count));
     SCATT_TRY(dW.alloc(ws * count));
@@ -223,17 +224,17 @@ int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* o
     SCATT_TRY(dP.alloc(ps * count));
     SCATT_TRY(dst.alloc(2 * (size_t)count));
     SCATT_TRY(dst.zero());
-    SCATT_TRY(dmag.alloc(4 * (size_t)count));
+    SCATT_TRY(dstat.alloc(words * count));
     SCATT_TRY(dbar.alloc(1));
     SCATT_TRY(dbar.zero());
     SCATT_CUDA_TRY(cudaMemcpy(dA.p, A, nn * count * sizeof(double), cudaMemcpyHostToDevice));
-    SCATT_TRY(dmag.zero());
+    SCATT_TRY(dstat.zero());
     std::vector<SymEntry> ent(count);
     const size_t T = sym_tiles_of(n);
     for (int b = 0; b < count; ++b) {
         double* P = dP.p + ps * b;
         ent[b] = SymEntry{dA.p + nn * b, dW.p + ws * b, P, P + T * SYM_TILE, P + 2 * T * SYM_TILE,
-                          dO.p + nn * b, dmag.p + 4 * b, dst.p + 2 * b, n, n};
+                          dO.p + nn * b, dstat.p + words * b, dst.p + 2 * b, n, n};
     }
     DevBuf<SymEntry> dent;
     SCATT_TRY(dent.upload(ent));
@@ -246,9 +247,9 @@ int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* o
     SCATT_CUDA_TRY(cudaMemcpy(st.data(), dst.p, st.size() * sizeof(int), cudaMemcpyDeviceToHost));
     if (status) std::memcpy(status, st.data(), st.size() * sizeof(int));
     if (mode) {
-        std::vector<unsigned long long> mg(4 * (size_t)count);
-        SCATT_CUDA_TRY(cudaMemcpy(mg.data(), dmag.p, mg.size() * sizeof(mg[0]), cudaMemcpyDeviceToHost));
-        for (int b = 0; b < count; ++b) mode[b] = (int)(mg[4 * (size_t)b + 3] & 0xffffffffu);
+        std::vector<unsigned> sw(words * count);
+        SCATT_CUDA_TRY(cudaMemcpy(sw.data(), dstat.p, sw.size() * sizeof(sw[0]), cudaMemcpyDeviceToHost));
+        for (int b = 0; b < count; ++b) mode[b] = (int)sw[words * b];
     }
     for (int b = 0; b < count; ++b)
         if (st[2 * b] != DEV_OK) {

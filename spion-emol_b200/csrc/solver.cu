@@ -230,13 +230,12 @@ __device__ __forceinline__ double* gacc_at(const BatchDev& b, const EnergyDev& d
     return (n & 1) ? d.G1 : d.G0;
 }
 
-// Entry of a symmetric inverse of order n (ld n throughout), its magnitudes and status cleared.
-__device__ __forceinline__ SymEntry sym_entry(double* A, double* W, double* panel, double* out,
-                                              unsigned long long* mag, int* status, int n) {
+// Entry of a symmetric inverse of order n (ld n throughout), its status cleared.
+__device__ __forceinline__ SymEntry sym_entry(double* A, double* W, double* panel, double* out, unsigned* stat,
+                                              int* status, int n) {
     const size_t T = sym_tiles_of(n);
-    mag[0] = mag[1] = mag[2] = mag[3] = 0;
     status[0] = status[1] = 0;
-    return SymEntry{A, W, panel, panel + T * SYM_TILE, panel + 2 * T * SYM_TILE, out, mag, status, n, n};
+    return SymEntry{A, W, panel, panel + T * SYM_TILE, panel + 2 * T * SYM_TILE, out, stat, status, n, n};
 }
 
 // Fills a chunk's GEMM and inverse entries, index j * count + e (pointer
@@ -249,6 +248,10 @@ __global__ void k_prepare(BatchDev b, bool symmetric) {
     dep_sync();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx <= SCHUR_CHUNK) b.barrier[idx] = 0;
+    // the records of both inverses' entries
+    const size_t words4 = 2 * (size_t)b.count * SCHUR_CHUNK * b.stat_stride / 4;
+    for (size_t u = idx; u < words4; u += (size_t)gridDim.x * blockDim.x)
+        reinterpret_cast<uint4*>(b.stat)[u] = make_uint4(0, 0, 0, 0);
     if (idx >= b.count * SCHUR_CHUNK) return;
     const int j = idx / b.count, e = idx % b.count;
     EnergyDev& d = b.ed[e];
@@ -279,7 +282,7 @@ __global__ void k_prepare(BatchDev b, bool symmetric) {
     b.gjS[idx] = GjEntry{S, d.Sw + j * b.sw_stride, sinv, d.sigS + (size_t)j * Np, d.ridS + (size_t)j * Np,
                          d.stS + 4 * j, symS ? 0 : Np, Np, Np, d.PS + j * b.ps_stride, d.sgS + (size_t)j * 4 * Np};
     if (symS) b.syS[idx] = sym_entry(S, d.Sw + j * b.sw_stride, d.PS + j * b.ps_stride, sinv,
-                                     b.mag + 4 * ((size_t)b.count * SCHUR_CHUNK + idx), d.stS + 4 * j, Np);
+                                     b.stat + ((size_t)b.count * SCHUR_CHUNK + idx) * b.stat_stride, d.stS + 4 * j, Np);
     else b.syS[idx].n = 0;
     b.gmT[idx] = exch ? GemmEntry{sinv, Bs, d.T, Np, Nf, Np, Np, b.Np_max, Np, 1.0, 0.0} : none;
     // F = Bs^T Sinv Bs is symmetric: lower tiles only, mirrored
@@ -295,7 +298,8 @@ __global__ void k_prepare(BatchDev b, bool symmetric) {
     const bool inv = n >= b.n_start;
     b.gjR[idx] = GjEntry{d.Ra, d.Rw, rinv, d.sigR, d.ridR, d.stR + 4 * j, inv && !symR ? Nt : 0, Nt, Nt, d.PR, d.sgR};
     if (inv) b.rargs[idx] = RArgs{sinv, d.T, d.F, Dinv_of(b, d, j), rinv_at(b, d, n - 1), Np, Nt, Nf, n < b.n_tr};
-    if (inv && symR) b.syR[idx] = sym_entry(d.Ra, d.Rw, d.PR, rinv, b.mag + 4 * (size_t)idx, d.stR + 4 * j, Nt);
+    if (inv && symR) b.syR[idx] = sym_entry(d.Ra, d.Rw, d.PR, rinv, b.stat + (size_t)idx * b.stat_stride,
+                                             d.stR + 4 * j, Nt);
     else b.syR[idx].n = 0;
 }
 
@@ -1512,7 +1516,7 @@ struct Scan {
     DevBuf<GemmEntry> gm;
     DevBuf<GjEntry> gj;
     DevBuf<SymEntry> sy;
-    DevBuf<unsigned long long> mag;
+    DevBuf<unsigned> stat;
     DevBuf<unsigned> barrier;
     DevBuf<RArgs> rargs;
     VBAt vb;                            // V/B at one step for the post stages
@@ -1671,13 +1675,14 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
     SCATT_TRY(sc.gm.alloc(7 * all));
     SCATT_TRY(sc.gj.alloc(2 * all));
     SCATT_TRY(sc.sy.alloc(2 * all));
-    SCATT_TRY(sc.mag.alloc(8 * all));
+    b.stat_stride = sym_stat_words(sc.Nt_cap);
+    SCATT_TRY(sc.stat.alloc(2 * all * b.stat_stride));
     SCATT_TRY(sc.barrier.alloc(SCHUR_CHUNK + 1));
     b.gmS = sc.gm.p; b.gmT = sc.gm.p + all; b.gmF = sc.gm.p + 2 * all; b.gmG = sc.gm.p + 3 * all;
     b.gmG3 = sc.gm.p + 5 * all; b.gmGA = sc.gm.p + 6 * all;
     b.gjR = sc.gj.p; b.gjS = sc.gj.p + all;
     b.syR = sc.sy.p; b.syS = sc.sy.p + all;
-    b.mag = sc.mag.p;
+    b.stat = sc.stat.p;
     b.barrier = sc.barrier.p;
     SCATT_TRY(sc.rargs.alloc(all));
     b.rargs = sc.rargs.p;
@@ -1870,6 +1875,8 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
             if (rinv[j]) {
                 if (sym_r) {
                     const int T = sym_tiles_of(sc.Nt_cap), nt = T * (T + 1) / 2;
+                    static std::atomic<unsigned long long> done{0};
+                    SCATT_TRY(sym_allow_smem(k_assemble_R_tiles, sizeof(SymDiagShared), done));
                     SCATT_TRY(run(k_assemble_R_tiles, dim3(count * nt), SYM_THREADS, sizeof(SymDiagShared), b, j, nt));
                 }
                 if (gen_r) SCATT_TRY(run(k_assemble_R, eg, TPB, 0, b, j));

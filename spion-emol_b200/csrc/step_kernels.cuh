@@ -100,10 +100,11 @@ struct BatchDev {
     // entry arrays written by k_prepare, SCHUR_CHUNK x slots each
     GemmEntry *gmS, *gmT, *gmF, *gmG, *gmG3, *gmGA;   // gmG: per step all C_n Sinv, then all -C_n T
     GjEntry *gjS, *gjR;
-    // the same inverses for the symmetric sweep, their magnitudes (4 words
-    // each), and the rescue's barrier counters: one per step's R, one for S
+    // the same inverses for the symmetric sweep, their records (R's entries
+    // first), and the rescue's barrier counters: one per step's R, one for S
     SymEntry *syS, *syR;
-    unsigned long long* mag;
+    unsigned* stat;
+    size_t stat_stride;     // words of one record
     unsigned* barrier;
     RArgs* rargs;           // SCHUR_CHUNK x slots
     size_t sw_stride, ps_stride;    // doubles of one Schur slot in Sw and PS

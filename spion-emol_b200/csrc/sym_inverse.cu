@@ -42,7 +42,7 @@ __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0
 // -acc into out (both triangles): tile rows from r0, columns from c0.
 __device__ __forceinline__ void store_out(const SymEntry& e, const double (&acc)[4][4], int r0, int c0, int wr, int wc,
                                           int lane) {
-    unsigned long long m = 0;
+    unsigned m = 0;
     const int g = lane >> 2, t = lane & 3;
 #pragma unroll
     for (int nb = 0; nb < 4; ++nb)
@@ -53,9 +53,9 @@ __device__ __forceinline__ void store_out(const SymEntry& e, const double (&acc)
             const double x = -acc[nb][v];
             e.out[r + (size_t)c * e.ldo] = x;
             if (r != c) e.out[c + (size_t)r * e.ldo] = x;
-            m = max(m, sym_bits(x));
+            m = max(m, sym_hi(x));
         }
-    sym_track_max(m, e.mag + 1);
+    sym_track(e, m, r0 / SYM_NB, c0 / SYM_NB, SYM_OF_X);
 }
 
 __global__ void __launch_bounds__(SYM_THREADS, 3)
@@ -101,8 +101,9 @@ constexpr size_t PANEL_SMEM = (SYM_TILE + PANEL_ROWS * SYM_NB) * sizeof(double);
 // elimination's 5.5e-13.  Where the tile's skew tells of it, one step by the
 // tile itself, L += (P - L A_KK) D, leaves the row residual at rounding
 // whatever kappa: 8.6e-13.  Only there: two products more of 64 x 64 a CTA.
-// Telling costs the inverse 2 % (order 1046: 28 matrices 1.763 -> 1.796 ms,
-// one 0.589 -> 0.601), as the pivot tile is kept and read again.
+// Telling costs the inverse 1 % (order 1046: 28 matrices 1.765 -> 1.781 ms, one
+// 0.597 -> 0.605), most of it the sums of |A_KK o D| at the end of each pivot
+// tile's chain.
 __global__ void __launch_bounds__(SYM_THREADS, 3)
 sym_panel_kernel(const SymEntry* entries, int K) {
     dep_sync();
@@ -117,16 +118,16 @@ sym_panel_kernel(const SymEntry* entries, int K) {
     const int wr = warp & 1, wc = warp >> 1;     // 16 rows, 16 columns
     if (i == K) {
         if (!last || half) return;
-        unsigned long long m = 0;
+        unsigned m = 0;
         for (int u = tid; u < SYM_TILE; u += SYM_THREADS) {
             const int r = u & 63, c = u >> 6;
             const int gr = K * SYM_NB + r, gc = K * SYM_NB + c;
             if (gr >= e.n || gc >= e.n) continue;
             const double x = e.D[r >= c ? sym_pos(r, c) : sym_pos(c, r)];
             e.out[gr + (size_t)gc * e.ldo] = x;
-            m = max(m, sym_bits(x));
+            m = max(m, sym_hi(x));
         }
-        sym_track_max(m, e.mag + 1);
+        sym_track(e, m, K, K, SYM_OF_X);
         return;
     }
     constexpr int HALF = PANEL_ROWS * SYM_NB;    // doubles
@@ -147,8 +148,10 @@ sym_panel_kernel(const SymEntry* entries, int K) {
     }
     for (int u = tid; u < SYM_TILE / 2; u += SYM_THREADS) cp16(Ds + 2 * u, e.D + 2 * u);
     cp_commit();
+    // read by one warp of the CTA: read by all, 272 warps at order 1046 queue for one line (0.5 us)
+    const bool skewed = tid < SYM_THREADS / 32 && sym_skew(e)[tid] > SYM_SKEW_MAX;
     cp_wait<0>();
-    __syncthreads();
+    const bool refine = __syncthreads_or(skewed);
     double acc[2][4];
 #pragma unroll
     for (int nb = 0; nb < 2; ++nb)
@@ -159,7 +162,7 @@ sym_panel_kernel(const SymEntry* entries, int K) {
     double* Mg = e.M + (size_t)i * SYM_TILE + half * HALF;
     for (int u = tid; u < HALF / 2; u += SYM_THREADS)
         reinterpret_cast<double2*>(Pg)[u] = reinterpret_cast<const double2*>(Ps)[u];
-    if (*sym_skew(e) > SYM_SKEW_MAX) {           // the same for the CTA
+    if (refine) {
         double res[2][4];                        // P - L A_KK
         const double2 *A2 = reinterpret_cast<const double2*>(sym_tile_of_D(e)), *D2 = reinterpret_cast<const double2*>(e.D);
         __syncthreads();                         // Ps and Ds are read by every warp above
@@ -188,7 +191,7 @@ sym_panel_kernel(const SymEntry* entries, int K) {
     }
     if (last) {
         // the inverse's tile (i, K) is -L_i
-        unsigned long long m = 0;
+        unsigned m = 0;
         const int g = lane >> 2, t = lane & 3;
 #pragma unroll
         for (int nb = 0; nb < 2; ++nb)
@@ -200,9 +203,9 @@ sym_panel_kernel(const SymEntry* entries, int K) {
                 const double x = -acc[nb][v];
                 e.out[r + (size_t)c * e.ldo] = x;
                 e.out[c + (size_t)r * e.ldo] = x;
-                m = max(m, sym_bits(x));
+                m = max(m, sym_hi(x));
             }
-        sym_track_max(m, e.mag + 1);
+        sym_track(e, m, i, K, SYM_OF_X);
     }
 #pragma unroll
     for (int nb = 0; nb < 2; ++nb)
@@ -324,7 +327,7 @@ sym_update_kernel(const SymEntry* entries, int count, int K, int nu, int ud) {
 #pragma unroll
             for (int v = 0; v < 4; ++v)
                 if ((v >> 1) * 8 < lim) m = max(m, sym_hi(acc[nb][v]));
-        sym_track_hi(m, sym_hi_of_schur(e));
+        sym_track(e, m, i, j, SYM_OF_SCHUR);
     }
     if (i == K + 1 && j == K + 1) {
         SymDiagShared& sh = *reinterpret_cast<SymDiagShared*>(smem);
@@ -332,11 +335,15 @@ sym_update_kernel(const SymEntry* entries, int count, int K, int nu, int ud) {
 #pragma unroll
         for (int nb = 0; nb < 4; ++nb)
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-                *reinterpret_cast<double2*>(sh.X + ((2 * wr + h) * 8 + 4 * wc + nb) * 64 + 2 * lane) =
-                    make_double2(acc[nb][2 * h], acc[nb][2 * h + 1]);
+            for (int h = 0; h < 2; ++h) {
+                const int R = 2 * wr + h, S = 4 * wc + nb;
+                const double2 x = make_double2(acc[nb][2 * h], acc[nb][2 * h + 1]);
+                *reinterpret_cast<double2*>(sh.X + (R * 8 + S) * 64 + 2 * lane) = x;
+                *reinterpret_cast<double2*>(sym_tile_of_D(e) + (R * 8 + S) * 64 + 2 * lane) = x;
+                if (R >= S) *reinterpret_cast<double2*>(sh.low + (R * (R + 1) / 2 + S) * 64 + 2 * lane) = x;
+            }
         __syncthreads();
-        sym_diag_invert(sh, sym_tile_of_D(e));
+        sym_diag_invert(sh);
         sym_diag_store(e, K + 1, sh);
         return;
     }
@@ -348,23 +355,14 @@ sym_update_kernel(const SymEntry* entries, int count, int K, int nu, int ud) {
                 make_double2(acc[nb][2 * h], acc[nb][2 * h + 1]);
 }
 
-int sym_attributes() {
-    int dev = 0;
-    SCATT_CUDA_TRY(cudaGetDevice(&dev));
-    static std::atomic<unsigned long long> done{0};
-    if (dev >= 0 && dev < 64 && (done.load() & (1ull << dev))) return SCATT_OK;
-    SCATT_CUDA_TRY(cudaFuncSetAttribute(sym_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_SMEM));
-    SCATT_CUDA_TRY(cudaFuncSetAttribute(sym_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)UPDATE_SMEM));
-    if (dev >= 0 && dev < 64) done.fetch_or(1ull << dev);
-    return SCATT_OK;
-}
-
 }  // namespace
 
 int sym_pack_batched(const SymEntry* entries_dev, int count, int nmax, cudaStream_t stream) {
     if (count <= 0 || nmax <= 0) return SCATT_OK;
     const int T = sym_tiles_of(nmax);
     const int nt = T * (T + 1) / 2;
+    static std::atomic<unsigned long long> done{0};
+    SCATT_TRY(sym_allow_smem(sym_pack_kernel, sizeof(SymDiagShared), done));
     SCATT_CUDA_TRY(launch_dep(sym_pack_kernel, count * nt, SYM_THREADS, sizeof(SymDiagShared), stream, entries_dev, count, nt));
     SCATT_COUNT_LAUNCH(1);
     return SCATT_OK;
@@ -376,7 +374,9 @@ int sym_sweep_batched(const SymEntry* entries_dev, int count, int nmax, cudaStre
         set_last_error("sym_sweep_batched: batch count exceeds 65535");
         return SCATT_ERR_ARG;
     }
-    SCATT_TRY(sym_attributes());
+    static std::atomic<unsigned long long> panel_done{0}, update_done{0};
+    SCATT_TRY(sym_allow_smem(sym_panel_kernel, PANEL_SMEM, panel_done));
+    SCATT_TRY(sym_allow_smem(sym_update_kernel, UPDATE_SMEM, update_done));
     const int T = sym_tiles_of(nmax), nu = T * (T - 1) / 2;
     for (int K = 0; K < T; ++K) {
         SCATT_CUDA_TRY(launch_dep(sym_panel_kernel, dim3(2 * T, count), SYM_THREADS, PANEL_SMEM, stream, entries_dev, K));

@@ -2,8 +2,12 @@
 // inverses grew (see sym_inverse.cu): one launch per batch, which returns at
 // once when no entry needs it.
 //
-// A sweep's error grows with g, the larger of max|D| / max|A^-1| and of the
-// Schur complements' largest element over A's.  The inverse takes a Newton step
+// A sweep's error grows with g, the larger of max|D_i| / max|A^-1| and of the
+// Schur complements' largest element over A's, each within a tile row i (over
+// the whole matrix, a large element of another block would hide the growth of
+// this one: blocks of delta I and I / delta beside one with a pivot tile of
+// delta = 1e-4 give 1, and an error of 1.5e-12 in that block), the largest of
+// the rows'.  The inverse takes a Newton step
 // X <- X (2 I - A X), two products over the whole grid for that entry alone,
 // which squares the relative error, where g > 3 (rare in a radial sweep, and
 // rarer the finer the grid), and a second one above g = 1e3.  Not elsewhere: the step leaves rounding of
@@ -101,7 +105,7 @@ __device__ __forceinline__ void sym_pivoted(const SymEntry& e, SymPivotShared& s
             const double v = A[r + (size_t)k * n];
             col[r] = v;
             if (step_of_row[r] < 0.0) {
-                const unsigned long long key = sym_bits(v);
+                const unsigned long long key = (unsigned long long)__double_as_longlong(fabs(v));
                 if (br == n || key > b) { b = key; br = r; }
             }
         }
@@ -182,21 +186,28 @@ sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, Source 
     for (int base = 0; base < count; base += SYM_RESCUE_LIST) {
         const int m = min(SYM_RESCUE_LIST, count - base);
         int any = 0;
-        for (int k = tid; k < m; k += SYM_THREADS) {
-            const SymEntry& e = entries[base + k];
-            int mode = 0;
-            if (e.n > 0) {
-                const double d = __longlong_as_double((long long)e.mag[0]);
-                const double x = __longlong_as_double((long long)e.mag[1]);
-                const double a = __hiloint2double((int)*sym_hi_of_A(e), 0), s = __hiloint2double((int)*sym_hi_of_schur(e), 0);
-                const double gr = fmax(d / x, s / a);
-                if (!isfinite(d) || !isfinite(x) || !isfinite(a) || !(x > 0.0) || !(gr <= 1e6)) mode = 3;
-                else if (e.n <= SYM_NB) mode = 0;           // one tile: pivoted throughout
-                else if (gr > 1e3) mode = 2;
-                else if (gr > 3.0) mode = 1;
-                if (blockIdx.x == 0) *sym_mode(e) = (unsigned)mode;
+        // four lanes an entry, every load of a lane in flight together: this stands in each step's chain
+        for (int k = tid >> 2; k < ((m + 7) & ~7); k += SYM_THREADS / 4) {
+            const int n = k < m ? entries[base + k].n : 0;
+            unsigned* stat = entries[base + min(k, m - 1)].stat;
+            double gr = 0.0;
+            bool bad = false;
+#pragma unroll 5
+            for (int i = tid & 3; i < sym_tiles_of(n); i += 4) {
+                const uint4 w = reinterpret_cast<const uint4*>(stat + SYM_STAT_HEAD)[i];
+                const double a = __hiloint2double((int)w.x, 0), s = __hiloint2double((int)w.y, 0);
+                const double d = __hiloint2double((int)w.z, 0), x = __hiloint2double((int)w.w, 0);
+                gr = fmax(gr, fmax(d / x, s / a));
+                bad |= !isfinite(a) || !isfinite(s) || !isfinite(d) || !isfinite(x) || !(a > 0.0) || !(x > 0.0);
             }
-            s_mode[k] = mode;
+            for (int o = 1; o <= 2; o <<= 1) gr = fmax(gr, __shfl_xor_sync(0xffffffffu, gr, o));
+            const unsigned quad = __ballot_sync(0xffffffffu, bad) >> (lane & ~3) & 15u;
+            // one tile is pivoted throughout
+            const int mode = n == 0 ? 0 : quad || !(gr <= 1e6) ? 3 : n <= SYM_NB ? 0 : gr > 1e3 ? 2 : gr > 3.0 ? 1 : 0;
+            if (k < m && (tid & 3) == 0) {
+                s_mode[k] = mode;
+                if (n > 0 && blockIdx.x == 0) stat[0] = (unsigned)mode;
+            }
             any |= mode;
         }
         if (!__syncthreads_or(any)) continue;

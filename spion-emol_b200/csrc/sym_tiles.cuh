@@ -11,6 +11,8 @@
 // taken in any order that both operands share, the operand pair too.
 #pragma once
 
+#include <cstddef>
+
 #include "common.cuh"
 
 namespace scatt {
@@ -26,10 +28,7 @@ struct SymEntry {
     double *P, *M;          // T tiles each: the pivot column block and its negated product with D
     double* D;              // the inverse of the pivot tile, the pivot tile itself, and sym_skew of the two
     double* out;            // n x n, ld ldo: the inverse, both triangles
-    // bit patterns of max |D| [0] and max |out| [1]; the high words of max |A|
-    // and of the largest element of the Schur complements [2]; how it was
-    // finished [3]
-    unsigned long long* mag;
+    unsigned* stat;         // sym_stat_words(n) words, zero before the sweep: [0] how it was finished, SYM_STAT_HEAD on sym_stat
     int* status;            // DeviceStatus, first failing column; zero before the sweep
     int n, ldo;
 };
@@ -47,19 +46,6 @@ __device__ __forceinline__ int sym_pos(int r, int c) {
     return (((r >> 3) << 3) + (c >> 3)) * 64 + ((r & 7) << 3) + (c & 7);
 }
 
-__device__ __forceinline__ unsigned long long sym_bits(double v) {
-    return (unsigned long long)__double_as_longlong(fabs(v));
-}
-
-// Largest of the warps' magnitudes into *dst (bit patterns: a NaN is larger than any number).
-__device__ __forceinline__ void sym_track_max(unsigned long long m, unsigned long long* dst) {
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
-        m = v > m ? v : m;
-    }
-    if ((threadIdx.x & 31) == 0) atomicMax(dst, m);
-}
-
 // Reciprocal by Newton-Raphson from the hardware's approximation (two steps:
 // relative error below 2^-50 from 2^-20); zero gives infinity.
 __device__ __forceinline__ double sym_rcp(double x) {
@@ -71,13 +57,26 @@ __device__ __forceinline__ double sym_rcp(double x) {
 
 constexpr int SYM_PANEL_LD = 10;   // doubles of a panel row: 16-byte rows apart by 5 mod 8, no bank conflicts
 
+__device__ __forceinline__ int sym_low_pos(int r, int c) {      // in SymDiagShared::low
+    return ((r >> 3) * ((r >> 3) + 1) / 2 + (c >> 3)) * 64 + ((r & 7) << 3) + (c & 7);
+}
 __device__ __forceinline__ unsigned sym_hi(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
-__device__ __forceinline__ unsigned* sym_hi_of_A(const SymEntry& e) { return reinterpret_cast<unsigned*>(e.mag + 2); }
-__device__ __forceinline__ unsigned* sym_hi_of_schur(const SymEntry& e) { return reinterpret_cast<unsigned*>(e.mag + 2) + 1; }
-__device__ __forceinline__ unsigned* sym_mode(const SymEntry& e) { return reinterpret_cast<unsigned*>(e.mag + 3); }
-__device__ __forceinline__ void sym_track_hi(unsigned m, unsigned* dst) {
+
+// What a sweep records of tile row i, as the high words of magnitudes (in
+// order as integers, a NaN above every number): the largest element of A's
+// tile row, of that row in any Schur complement, of the pivot tile's inverse
+// D_i, and of the inverse's tile row.
+enum SymStat { SYM_OF_A = 0, SYM_OF_SCHUR = 1, SYM_OF_D = 2, SYM_OF_X = 3 };
+constexpr int SYM_STAT_HEAD = 4;
+__host__ __device__ inline size_t sym_stat_words(int n) { return SYM_STAT_HEAD + 4 * (size_t)sym_tiles_of(n); }
+__device__ __forceinline__ unsigned* sym_stat(const SymEntry& e, int i, SymStat q) { return e.stat + SYM_STAT_HEAD + 4 * i + q; }
+// A warp's part of an element block of tile (i, j): it counts for both tile rows.
+__device__ __forceinline__ void sym_track(const SymEntry& e, unsigned m, int i, int j, SymStat q) {
     m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) atomicMax(dst, m);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(sym_stat(e, i, q), m);
+        if (i != j) atomicMax(sym_stat(e, j, q), m);
+    }
 }
 
 struct SymDiagShared {
@@ -88,11 +87,14 @@ struct SymDiagShared {
     unsigned long long took[2];                  // those of the last panel, by parity
     int prow[SYM_NB];                            // row of each step's pivot
     int krow[SYM_NB];                            // step at which each row was the pivot
-    double skew[SYM_THREADS / 32];               // each warp's part of sym_skew
+    alignas(16) double low[36 * 64];             // the tile's sub-blocks (R, C), R >= C, at R (R + 1) / 2 + C
 };
 
+static_assert(offsetof(SymDiagShared, panel) % 16 == 0 && offsetof(SymDiagShared, row) % 16 == 0 &&
+              offsetof(SymDiagShared, low) % 16 == 0, "read and written in 16-byte pieces");
+
 // Pivot tiles whose largest column sum of |A_ij D_ij| (A the tile, D its
-// inverse) is above this have their rows L = P D refined (sym_panel_kernel).
+// inverse; sym_skew holds the largest of each warp's columns) is above this have their rows L = P D refined (sym_panel_kernel).
 // The sum is 1 for a diagonal or a well-conditioned dominant tile, does not
 // change when rows and columns are scaled alike (a tile graded by its
 // centrifugal terms has a condition number of 1e3 and a sum below 1.4), and
@@ -225,8 +227,7 @@ __device__ __forceinline__ void sym_diag_panel(SymDiagShared& sh, int c, int lan
 // applies it to its own block by DMMAs and goes on to the next panel, and the
 // other warps apply it meanwhile.  Rows are not moved: row p_k of step k ends
 // as row k of the inverse, whose column p_j sits in column j.  The result is
-// symmetrised and left in sh.X; the tile itself goes to `tile`, and sh.skew
-// gets the column sums of SYM_SKEW_MAX.
+// symmetrised and left in sh.X.
 //
 // Bound by the chain of 64 pivots, each of which stays inside a warp.  A form
 // with the rows spread over the CTA, and one or two barriers a pivot, took
@@ -235,7 +236,7 @@ __device__ __forceinline__ void sym_diag_panel(SymDiagShared& sh, int c, int lan
 // order) the growth of the intermediate inverses reaches 1e3 to 1e4 and the
 // solver's results lose one to four digits; with it the growth seen is mostly
 // below 2.
-__device__ __forceinline__ void sym_diag_invert(SymDiagShared& sh, double* tile) {
+__device__ __forceinline__ void sym_diag_invert(SymDiagShared& sh) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     // a lane's element (r, c) of the warp's u-th 8 x 4 patch, and its mirror image: at most four-way conflicts
@@ -252,12 +253,6 @@ __device__ __forceinline__ void sym_diag_invert(SymDiagShared& sh, double* tile)
     }
     if (tid == 0) sh.used = 0;
     __syncthreads();
-    // every warp its own column block, which no other changes before the first panel is applied
-#pragma unroll
-    for (int R = 0; R < 8; ++R) {
-        const int off = (R * 8 + warp) * 64 + 2 * lane;
-        *reinterpret_cast<double2*>(tile + off) = *reinterpret_cast<const double2*>(sh.X + off);
-    }
     // block <- (block with the panel's pivot rows zeroed) + panel * (pivot rows of the block)
     auto apply = [&](int c) {
         const double* pan = sh.panel[c & 1];
@@ -298,33 +293,15 @@ __device__ __forceinline__ void sym_diag_invert(SymDiagShared& sh, double* tile)
         __syncthreads();
         if (warp != c && warp != c + 1) apply(c);
     }
-    double v[16];                                // the tile's elements, then the inverse's
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-        int r, c;
-        patch(u, r, c);
-        v[u] = __ldcg(tile + sym_pos(r, c));
-    }
     __syncthreads();
-    // inverse(r, c) = X(p_r, step of c), symmetrised; a lane's patches lie in two columns, by parity of u
-    double sum[2] = {0.0, 0.0};
+    // inverse(r, c) = X(p_r, step of c), symmetrised
+    double v[16];
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
         int r, c;
         patch(u, r, c);
-        const double x = 0.5 * (sh.X[sym_pos(sh.prow[r], sh.krow[c])] + sh.X[sym_pos(sh.prow[c], sh.krow[r])]);
-        sum[u & 1] += fabs(x * v[u]);
-        v[u] = x;
+        v[u] = 0.5 * (sh.X[sym_pos(sh.prow[r], sh.krow[c])] + sh.X[sym_pos(sh.prow[c], sh.krow[r])]);
     }
-#pragma unroll
-    for (int o = 16; o >= 4; o >>= 1) {
-        sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], o);
-        sum[1] += __shfl_xor_sync(0xffffffffu, sum[1], o);
-    }
-    sum[0] = fmax(sum[0], sum[1]);
-#pragma unroll
-    for (int o = 2; o >= 1; o >>= 1) sum[0] = fmax(sum[0], __shfl_xor_sync(0xffffffffu, sum[0], o));
-    if (lane == 0) sh.skew[warp] = sum[0];
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
@@ -360,28 +337,41 @@ __device__ __forceinline__ void sym_tile_mma(double (&acc)[4][4], const double* 
 }
 
 // Writes the inverse of pivot tile K (in sh.X) to D and, negated, to the
-// matrix, and tracks its largest element inside the order.
+// matrix, tracks its largest element inside the order, and writes sym_skew from
+// the tile in sh.low.
 __device__ __forceinline__ void sym_diag_store(const SymEntry& e, int K, const SymDiagShared& sh) {
     double2* D = reinterpret_cast<double2*>(e.D);
     double2* W = reinterpret_cast<double2*>(e.W + sym_tile_index(K, K) * SYM_TILE);
     const double2* X = reinterpret_cast<const double2*>(sh.X);
-    unsigned long long m = 0;
-    for (int u = threadIdx.x; u < SYM_TILE / 2; u += SYM_THREADS) {
+    unsigned m = 0;
+    double s0 = 0.0, s1 = 0.0;               // of the lane's two columns
+    const int lane = threadIdx.x & 31, C = threadIdx.x >> 5;
+#pragma unroll
+    for (int R = 0; R < 8; ++R) {
+        const int u = threadIdx.x + R * SYM_THREADS;
         const double2 v = X[u];
+        const double* low = sh.low + (R >= C ? R * (R + 1) / 2 + C : C * (C + 1) / 2 + R) * 64;
+        const int g = lane >> 2, t = lane & 3;
+        s0 += fabs(v.x * low[R >= C ? 2 * lane : 16 * t + g]);
+        s1 += fabs(v.y * low[R >= C ? 2 * lane + 1 : 16 * t + 8 + g]);
         D[u] = v;
         W[u] = make_double2(-v.x, -v.y);
         // pair u: sub-block u / 32, row (u % 32) / 4
         const int row = K * SYM_NB + (u >> 8) * 8 + ((u & 31) >> 2);
         const int col = K * SYM_NB + ((u >> 5) & 7) * 8 + (u & 3) * 2;
-        if (row < e.n && col < e.n) m = max(m, sym_bits(v.x));
-        if (row < e.n && col + 1 < e.n) m = max(m, sym_bits(v.y));
+        if (row < e.n && col < e.n) m = max(m, sym_hi(v.x));
+        if (row < e.n && col + 1 < e.n) m = max(m, sym_hi(v.y));
     }
-    sym_track_max(m, e.mag);
-    if (threadIdx.x == 0) {
-        double s = sh.skew[0];
-        for (int w = 1; w < SYM_THREADS / 32; ++w) s = fmax(s, sh.skew[w]);
-        *sym_skew(e) = s;
+    sym_track(e, m, K, K, SYM_OF_D);
+#pragma unroll
+    for (int o = 16; o >= 4; o >>= 1) {
+        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
     }
+    s0 = fmax(s0, s1);
+#pragma unroll
+    for (int o = 2; o >= 1; o >>= 1) s0 = fmax(s0, __shfl_xor_sync(0xffffffffu, s0, o));
+    if (lane == 0) sym_skew(e)[C] = s0;
 }
 
 // Packs tile t of entry e from elem(row, column, inside) (the element of a
@@ -412,12 +402,17 @@ __device__ __forceinline__ void sym_pack_tile(const SymEntry& e, int t, SymDiagS
         const int gi = i * SYM_NB + r, gj = j * SYM_NB + c;
         const bool in = gi < e.n && gj < e.n;
         if (in) m = max(m, sym_hi(v[u]));
-        W[sym_pos(r, c)] = in ? v[u] : gi == gj ? 1.0 : 0.0;
+        const double x = in ? v[u] : gi == gj ? 1.0 : 0.0;
+        W[sym_pos(r, c)] = x;
+        if (first) {
+            sym_tile_of_D(e)[sym_pos(r, c)] = x;
+            if (r >> 3 >= c >> 3) sh.low[sym_low_pos(r, c)] = x;
+        }
     }
-    sym_track_hi(m, sym_hi_of_A(e));
+    sym_track(e, m, i, j, SYM_OF_A);
     if (first) {
         __syncthreads();
-        sym_diag_invert(sh, sym_tile_of_D(e));
+        sym_diag_invert(sh);
         sym_diag_store(e, 0, sh);
     }
 }
@@ -437,7 +432,18 @@ __device__ __forceinline__ void sym_pack_index(int bid, int count, int nt, int& 
 // Sweeps a packed batch (pivot tile 0 already inverted) to the inverses, all
 // entries of order <= nmax; entries of order 0 are skipped.
 int sym_sweep_batched(const SymEntry* entries_dev, int count, int nmax, cudaStream_t stream);
-// Packs full symmetric matrices (entry.A) for sym_sweep_batched; mag and status must be zero.
+// Packs full symmetric matrices (entry.A) for sym_sweep_batched; stat and status must be zero.
 int sym_pack_batched(const SymEntry* entries_dev, int count, int nmax, cudaStream_t stream);
+
+// Once per device: the dynamic shared memory that `kernel` may ask for; `done` has a bit per device.
+template <class... P>
+int sym_allow_smem(void (*kernel)(P...), size_t bytes, std::atomic<unsigned long long>& done) {
+    int dev = 0;
+    SCATT_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && (done.load() & (1ull << dev))) return SCATT_OK;
+    SCATT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (dev >= 0 && dev < 64) done.fetch_or(1ull << dev);
+    return SCATT_OK;
+}
 
 }  // namespace scatt

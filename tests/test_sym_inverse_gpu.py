@@ -136,3 +136,26 @@ def test_dominant_directions(n, kind):
         err = lambda y: np.linalg.norm(y @ b - t) / np.linalg.norm(t)  # noqa: E731
         # the floor: rounding of the products X b themselves
         assert err(x) <= 10.0 * err(g) + 1e-15, (c, err(x), err(g))
+
+
+@pytest.mark.parametrize("n", [256, 300])
+@pytest.mark.parametrize("delta,want", [(1e-2, 1), (1e-4, 2), (1e-6, 2)])
+def test_growth_in_one_block_only(n, delta, want):
+    """The nearly singular leading block beside uncoupled blocks delta I and
+    I / delta: these hold the largest element of A and of its inverse, so that
+    only a record per tile row sees the first block's growth.  Its own part of
+    the inverse is held to rounding (the sweep alone leaves eps / delta)."""
+    rng = np.random.default_rng(9)
+    A = np.zeros((1, n, n))
+    A[0, :128, :128] = symmetric(rng, 1, 128)[0]
+    A[0, :64, :64] = delta * np.diag(1.0 + rng.random(64))
+    A[0, :64, 64:128] = np.linalg.qr(rng.standard_normal((64, 64)))[0]
+    A[0, 64:128, :64] = A[0, :64, 64:128].T
+    i = np.arange(128, n)
+    A[0, i, i] = np.where(i < 192, delta, 1.0 / delta)
+    X, st, mode = _lib.inverse_symmetric_batched(A)
+    assert st[0, 0] == 0 and mode[0] == want
+    ref = np.linalg.inv(A[0, :128, :128])
+    kappa = np.linalg.cond(A[0, :128, :128])
+    assert np.max(np.abs(X[0, :128, :128] - ref)) <= 1e-13 * max(10.0, kappa) * np.max(np.abs(ref))
+    assert np.max(np.abs(X[0, i, i] * A[0, i, i] - 1.0)) <= 1e-14
