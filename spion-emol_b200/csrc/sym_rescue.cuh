@@ -20,8 +20,11 @@
 //              1200    21      3.9e-11  7.7e-16  8.4e-16  1.1e-14
 //              15      1.4e3   7.7e-13  7.0e-15  3.9e-13  7.4e-13
 //   median     1       20      7e-16             6e-16
-// Past g = 1e6, and on zero and non-finite pivots, to report them, the entry
-// takes a pivoted elimination by one CTA: slow, and not met in normal running.
+// The steps' changes tell whether they converge: a step more is taken while
+// one is above 1e-6, three at most.  Where they grow instead (condition numbers
+// past 1e9 beside a growth of 1e5), past g = 1e6, and on zero and non-finite
+// pivots, to report them, the entry takes a pivoted elimination by one CTA:
+// slow, and not met in normal running.
 #pragma once
 
 #include "sym_tiles.cuh"
@@ -219,7 +222,8 @@ sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, Source 
             const int n = e.n, T = sym_tiles_of(n);
             source(base + k, e, blockIdx.x * SYM_THREADS + tid, gridDim.x * SYM_THREADS);
             alive = sym_grid_barrier(barrier, turn);
-            for (int step = 0; step < mode && alive; ++step) {
+            double last = INFINITY;                 // change of the step before
+            for (int step = 0; alive; ++step) {
                 for (int half = 0; half < 2 && alive; ++half) {
                     // W = A X, then the second half of W = X W (A and X are symmetric)
                     for (int u = blockIdx.x; u < T * T; u += gridDim.x) {
@@ -241,18 +245,35 @@ sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, Source 
                 }
                 if (!alive) break;
                 const double* Z = e.W + (size_t)n * n;
+                double ch = 0.0;                    // largest change over the smaller of its two tile rows' maxima
                 for (long u = blockIdx.x * (long)SYM_THREADS + tid; u < (long)n * n; u += (long)gridDim.x * SYM_THREADS) {
                     const int r = (int)(u % n), c = (int)(u / n);
                     if (c > r) continue;
                     const double z = 0.5 * (Z[r + (size_t)c * n] + Z[c + (size_t)r * n]);
-                    const double x = 2.0 * e.out[r + (size_t)c * e.ldo] - z;
+                    const double x0 = e.out[r + (size_t)c * e.ldo], x = 2.0 * x0 - z;
                     e.out[r + (size_t)c * e.ldo] = x;
                     e.out[c + (size_t)r * e.ldo] = x;
+                    const unsigned row = min(*sym_stat(e, r / SYM_NB, SYM_OF_X), *sym_stat(e, c / SYM_NB, SYM_OF_X));
+                    const double q = fabs(x - x0) / __hiloint2double((int)row, 0);
+                    ch = q <= ch ? ch : q;          // a NaN stays
                 }
+                const unsigned hi = __reduce_max_sync(0xffffffffu, sym_hi(ch));
+                if (lane == 0) atomicMax(e.stat + 1 + step, hi);
                 alive = sym_grid_barrier(barrier, turn);
+                ch = __hiloint2double((int)__ldcg(e.stat + 1 + step), 0);
+                // not contracting: the elimination below (every CTA decides the same)
+                if (!(ch <= 0.1) || (ch > 1e-6 && (ch > last || step + 1 == SYM_STEPS))) {
+                    __syncthreads();                // s_mode[k] has been read
+                    if (tid == 0) s_mode[k] = 3;
+                    if (blockIdx.x == 0 && tid == 0) e.stat[0] = 3;
+                    break;
+                }
+                if (step + 1 >= mode && ch <= 1e-6) break;
+                last = ch;
             }
             if (!alive && blockIdx.x == 0 && tid == 0) e.status[0] = DEV_NONFINITE;
         }
+        __syncthreads();
         // pivoted eliminations, one CTA each
         for (int k = 0; k < m; ++k) {
             if (s_mode[k] != 3 || (base + k) % (int)gridDim.x != (int)blockIdx.x) continue;

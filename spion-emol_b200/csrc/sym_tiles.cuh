@@ -28,7 +28,8 @@ struct SymEntry {
     double *P, *M;          // T tiles each: the pivot column block and its negated product with D
     double* D;              // the inverse of the pivot tile, the pivot tile itself, and sym_skew of the two
     double* out;            // n x n, ld ldo: the inverse, both triangles
-    unsigned* stat;         // sym_stat_words(n) words, zero before the sweep: [0] how it was finished, SYM_STAT_HEAD on sym_stat
+    unsigned* stat;         // sym_stat_words(n) words, zero before the sweep: [0] how it was finished, [1 ..] SYM_STEPS Newton
+                            // steps' changes, SYM_STAT_HEAD on sym_stat
     int* status;            // DeviceStatus, first failing column; zero before the sweep
     int n, ldo;
 };
@@ -67,7 +68,7 @@ __device__ __forceinline__ unsigned sym_hi(double v) { return (unsigned)__double
 // tile row, of that row in any Schur complement, of the pivot tile's inverse
 // D_i, and of the inverse's tile row.
 enum SymStat { SYM_OF_A = 0, SYM_OF_SCHUR = 1, SYM_OF_D = 2, SYM_OF_X = 3 };
-constexpr int SYM_STAT_HEAD = 4;
+constexpr int SYM_STEPS = 3, SYM_STAT_HEAD = 1 + SYM_STEPS;
 __host__ __device__ inline size_t sym_stat_words(int n) { return SYM_STAT_HEAD + 4 * (size_t)sym_tiles_of(n); }
 __device__ __forceinline__ unsigned* sym_stat(const SymEntry& e, int i, SymStat q) { return e.stat + SYM_STAT_HEAD + 4 * i + q; }
 // A warp's part of an element block of tile (i, j): it counts for both tile rows.

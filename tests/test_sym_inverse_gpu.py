@@ -159,3 +159,31 @@ def test_growth_in_one_block_only(n, delta, want):
     kappa = np.linalg.cond(A[0, :128, :128])
     assert np.max(np.abs(X[0, :128, :128] - ref)) <= 1e-13 * max(10.0, kappa) * np.max(np.abs(ref))
     assert np.max(np.abs(X[0, i, i] * A[0, i, i] - 1.0)) <= 1e-14
+
+
+@pytest.mark.parametrize("lam", [1e-6, 1e-8, 1e-9, 1e-10, 1e-11])
+def test_newton_steps_that_do_not_converge(lam):
+    """A nearly singular leading block (growth 2e5) in a matrix of condition
+    about 5 / lam: past 1e9 the Newton steps run away, and the entry has to end
+    in the pivoted elimination.  Held to ten times what rounding of A does to
+    the inverse, kappa eps."""
+    n = 200
+    rng = np.random.default_rng(5)
+    A = symmetric(rng, 1, n)
+    A[0, :64, :64] = 2e-6 * np.eye(64)
+    A[0, :64, 64:128] = A[0, 64:128, :64] = np.eye(64)
+    A[0, :64, 128:] = A[0, 128:, :64] = 0.0
+    A[0, 64:128, 128:] = 0.5 / 8.0 * rng.standard_normal((64, n - 128))
+    A[0, 128:, 64:128] = A[0, 64:128, 128:].T
+    v = np.zeros(n)
+    v[128:] = rng.standard_normal(n - 128)
+    v /= np.linalg.norm(v)
+    # A + t v v^T is singular at t = -1 / (v^T A^-1 v)
+    A[0] -= (1.0 + lam) / (v @ np.linalg.solve(A[0], v)) * np.outer(v, v)
+    A[0] = 0.5 * (A[0] + A[0].T)
+    X, st, mode = _lib.inverse_symmetric_batched(A)
+    assert st[0, 0] == 0
+    b = rng.standard_normal((n, 4))
+    t = _solutions(A[0], np.linalg.inv(A[0]), b)
+    kappa = np.linalg.cond(A[0])
+    assert np.linalg.norm(X[0] @ b - t) <= 10.0 * kappa * 2.2e-16 * np.linalg.norm(t), (mode[0], kappa)
