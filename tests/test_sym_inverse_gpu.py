@@ -187,3 +187,32 @@ def test_newton_steps_that_do_not_converge(lam):
     t = _solutions(A[0], np.linalg.inv(A[0]), b)
     kappa = np.linalg.cond(A[0])
     assert np.linalg.norm(X[0] @ b - t) <= 10.0 * kappa * 2.2e-16 * np.linalg.norm(t), (mode[0], kappa)
+
+
+@pytest.mark.parametrize("n", [1, 64, 200])
+def test_reciprocals_of_pivots(n):
+    """Diagonal matrices: the inverse is the pivots' reciprocals, to half an
+    ulp (and the 2^-27 of one that the Newton steps leave)."""
+    rng = np.random.default_rng(n)
+    d = np.ldexp(1.0 + rng.random((40, n)), rng.integers(-4, 5, size=(40, n)) + rng.integers(-900, 900, size=(40, 1)))
+    d *= np.where(rng.random((40, n)) < 0.5, -1.0, 1.0)
+    A = np.zeros((40, n, n))
+    i = np.arange(n)
+    A[:, i, i] = d
+    X, st, mode = _lib.inverse_symmetric_batched(A)
+    assert np.all(st == 0) and np.all(mode == 0)
+    y = X[:, i, i].astype(np.longdouble)
+    assert np.max(np.abs(y * d.astype(np.longdouble) - 1)) <= np.longdouble(2.0) ** -53 * (1 + 2.0 ** -9)
+    assert np.count_nonzero(X) == d.size
+
+
+@pytest.mark.parametrize("value", [2.0 ** -1023, 1.5 * 2.0 ** -1023, 2.0 ** 1022, 1.25 * 2.0 ** 1022, 1.7 * 2.0 ** 1023])
+@pytest.mark.parametrize("at", [0, 40, 120])
+def test_pivots_outside_the_reciprocal(value, at):
+    A = np.eye(130)[None].copy()
+    A[0, at, at] = value
+    X, st, _ = _lib.inverse_symmetric_batched(A)
+    assert st[0, 0] == 0
+    want = np.eye(130)
+    want[at, at] = 1.0 / value                      # a subnormal number for the last two
+    assert np.all(np.abs(X[0] - want) <= np.where(want == 1.0 / value, np.spacing(want), 0.0))
