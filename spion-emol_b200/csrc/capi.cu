@@ -213,7 +213,7 @@ int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* o
     SCATT_TRY(require_device());
     const size_t nn = (size_t)n * n, al = 31;
     const size_t ws = (sym_work_doubles(n) + al) & ~al, ps = sym_panel_doubles(n);
-    DevBuf<double> dA, dW, dO, dP;
+    DevBuf<double> dA, dW, dO, dP, dS;
     DevBuf<int> dst;
     DevBuf<unsigned> dstat;
     const size_t words = sym_stat_words(n);
@@ -222,6 +222,7 @@ int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* o
     SCATT_TRY(dW.alloc(ws * count));
     SCATT_TRY(dO.alloc(nn * count));
     SCATT_TRY(dP.alloc(ps * count));
+    SCATT_TRY(dS.alloc(sym_scratch_doubles(n)));
     SCATT_TRY(dst.alloc(2 * (size_t)count));
     SCATT_TRY(dst.zero());
     SCATT_TRY(dstat.alloc(words * count));
@@ -240,7 +241,7 @@ int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* o
     SCATT_TRY(dent.upload(ent));
     SCATT_TRY(sym_pack_batched(dent.p, count, n, 0));
     SCATT_TRY(sym_sweep_batched(dent.p, count, n, 0));
-    SCATT_TRY(sym_rescue_batched(dent.p, count, dbar.p, 0));
+    SCATT_TRY(sym_rescue_batched(dent.p, count, dbar.p, dS.p, 0));
     SCATT_CUDA_TRY(cudaDeviceSynchronize());
     SCATT_CUDA_TRY(cudaMemcpy(out, dO.p, nn * count * sizeof(double), cudaMemcpyDeviceToHost));
     std::vector<int> st(2 * count);

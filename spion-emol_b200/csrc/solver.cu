@@ -1423,7 +1423,11 @@ int ensure_stab(Context& ctx, const scatt_solve_opts& o, int l_cont, const doubl
 
 // Doubles of the panel buffers of one inverse of order n: the Gauss-Jordan
 // windows (four, with the look-ahead) or the symmetric sweep's P, M and D.
-size_t panel_doubles(int n) { return std::max((size_t)4 * GJ_WINDOW_MAX * n, sym_panel_doubles(n)); }
+size_t panel_doubles(int n) {
+    return std::max((size_t)4 * GJ_WINDOW_MAX * n, n > SYM_NB ? sym_panel_doubles(n) : 0);
+}
+// Doubles of its work buffer: n x n for the Gauss-Jordan, or the sweep's tiles.
+size_t work_doubles(int n) { return std::max((size_t)n * n, n > SYM_NB ? sym_work_doubles(n) : 0); }
 
 // Device doubles of one slot sized for (Np, Nt): the chunk's Schur slots,
 // the W^-1 blocks, the R ping-pong buffers, the dipole rows, the asymptotic
@@ -1435,8 +1439,8 @@ size_t slot_doubles(const BatchDev& b, int Np, int Nt, int l_cont, bool keep_win
     const int nslots = b.N - b.n_s + 1;
     auto al = [](size_t c) { return (c + 31) & ~size_t(31); };
     const size_t np2 = (size_t)Np * Np, nt2 = (size_t)Nt * Nt;
-    const size_t base = 2 * al(SCHUR_CHUNK * np2) + al(SCHUR_CHUNK * al(sym_work_doubles(Np))) +
-                        al((size_t)Np * b.Nf) + al((size_t)b.Nf * b.Nf) + 3 * al(nt2) + al(sym_work_doubles(Nt)) +
+    const size_t base = 2 * al(SCHUR_CHUNK * np2) + al(SCHUR_CHUNK * al(work_doubles(Np))) +
+                        al((size_t)Np * b.Nf) + al((size_t)b.Nf * b.Nf) + 3 * al(nt2) + al(work_doubles(Nt)) +
                         2 * al((size_t)b.Krows * Nt) + al(SCHUR_CHUNK * al(panel_doubles(Np))) + al(panel_doubles(Nt));
     if (keep_window) return base + al((size_t)nslots * nt2) + 2 * al((size_t)nslots * np2);
     return base + 2 * al((size_t)2 * Np * Nt) + al((size_t)b.nfit * 2 * Np) + al((size_t)8 * (l_cont + 1));
@@ -1518,6 +1522,7 @@ struct Scan {
     DevBuf<SymEntry> sy;
     DevBuf<unsigned> stat;
     DevBuf<unsigned> barrier;
+    DevBuf<double> scratch;
     DevBuf<RArgs> rargs;
     VBAt vb;                            // V/B at one step for the post stages
     std::vector<PostBufs> P;            // gs energies
@@ -1591,7 +1596,7 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
     sc.nfit = sc.ne_fit - b.n_s + 1;
     b.count = slots;
     b.ngroups = ngroups;
-    b.sw_stride = (sym_work_doubles(sc.Np_cap) + 31) & ~size_t(31);
+    b.sw_stride = (work_doubles(sc.Np_cap) + 31) & ~size_t(31);
     b.ps_stride = (panel_doubles(sc.Np_cap) + 31) & ~size_t(31);
     const int K = b.Krows, Nf = b.Nf;
     // ---- slot arena
@@ -1616,7 +1621,7 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
         d.T = take((size_t)sc.Np_cap * Nf);
         d.F = take((size_t)Nf * Nf);
         d.Ra = take(nt2);
-        d.Rw = take(sym_work_doubles(sc.Nt_cap));
+        d.Rw = take(work_doubles(sc.Nt_cap));
         d.Rinv0 = take(nt2);
         d.Rinv1 = take(nt2);
         d.G0 = take((size_t)K * sc.Nt_cap);
@@ -1678,6 +1683,7 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
     b.stat_stride = sym_stat_words(sc.Nt_cap);
     SCATT_TRY(sc.stat.alloc(2 * all * b.stat_stride));
     SCATT_TRY(sc.barrier.alloc(SCHUR_CHUNK + 1));
+    SCATT_TRY(sc.scratch.alloc(sym_scratch_doubles(sc.Nt_cap)));      // S and R are rescued one after the other
     b.gmS = sc.gm.p; b.gmT = sc.gm.p + all; b.gmF = sc.gm.p + 2 * all; b.gmG = sc.gm.p + 3 * all;
     b.gmG3 = sc.gm.p + 5 * all; b.gmGA = sc.gm.p + 6 * all;
     b.gjR = sc.gj.p; b.gjS = sc.gj.p + all;
@@ -1855,7 +1861,7 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
         if (sym_s) {
             SCATT_TRY(sym_pack_batched(b.syS, count * SCHUR_CHUNK, sc.Np_cap, s));
             SCATT_TRY(sym_sweep_batched(b.syS, count * SCHUR_CHUNK, sc.Np_cap, s));
-            SCATT_TRY(sym_rescue_batched(b.syS, count * SCHUR_CHUNK, b.barrier + SCHUR_CHUNK, s));
+            SCATT_TRY(sym_rescue_batched(b.syS, count * SCHUR_CHUNK, b.barrier + SCHUR_CHUNK, sc.scratch.p, s));
         }
         if (gen_s) SCATT_TRY(gj_inverse_selected(b.gjS, count * SCHUR_CHUNK, gen_Np, true, s, true));
         // ---- the R-ratio recurrence over the chunk's steps
@@ -1889,7 +1895,7 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                 }
                 if (sym_r) {
                     SCATT_TRY(sym_sweep_batched(b.syR + at, count, sc.Nt_cap, s));
-                    SCATT_TRY(sym_rescue_launch(b.syR + at, count, b.barrier + j, RSource{b, j}, s));
+                    SCATT_TRY(sym_rescue_launch(b.syR + at, count, b.barrier + j, sc.scratch.p, RSource{b, j}, s));
                 }
                 if (gen_r) SCATT_TRY(gj_inverse_selected(b.gjR + at, count, gen_Nt, true, s, true));
                 if (sample) {
@@ -2558,7 +2564,7 @@ int slots_that_fit(Context& ctx, const scatt_solve_opts& o, int l_cap, int group
     const size_t per = 8 * (slot_doubles(b, Np, Nt, l_cap, o.keep_window != 0) +
                             post_doubles(b, Np, Nt, l_cap, nfit, t.n_occ)) +
                        4 * slot_ints(Np, Nt);
-    const size_t fixed = 8 * group_doubles(b) * (size_t)groups + (64u << 20);
+    const size_t fixed = 8 * (group_doubles(b) * (size_t)groups + sym_scratch_doubles(Nt)) + (64u << 20);
     const size_t avail = (size_t)(0.85 * freeb) > fixed ? (size_t)(0.85 * freeb) - fixed : 0;
     *out = (int)std::max<size_t>(1, avail / std::max<size_t>(per, 1));
     return SCATT_OK;

@@ -397,8 +397,8 @@ struct KeptSource {
 };
 }  // namespace
 
-int sym_rescue_batched(const SymEntry* entries_dev, int count, unsigned* barrier, cudaStream_t stream) {
-    return sym_rescue_launch(entries_dev, count, barrier, KeptSource{}, stream);
+int sym_rescue_batched(const SymEntry* entries_dev, int count, unsigned* barrier, double* scratch, cudaStream_t stream) {
+    return sym_rescue_launch(entries_dev, count, barrier, scratch, KeptSource{}, stream);
 }
 
 }  // namespace scatt

@@ -178,7 +178,7 @@ constexpr int SYM_RESCUE_LIST = 256;          // entries looked at in one pass
 // one CTA: passes over the list are not ordered between the CTAs.
 template <class Source>
 __global__ void __launch_bounds__(SYM_THREADS, 1)
-sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, Source source) {
+sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, double* scratch, Source source) {
     extern __shared__ double smem[];
     __shared__ int s_mode[SYM_RESCUE_LIST];
     __shared__ SymPivotShared s_piv;
@@ -225,13 +225,13 @@ sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, Source 
             double last = INFINITY;                 // change of the step before
             for (int step = 0; alive; ++step) {
                 for (int half = 0; half < 2 && alive; ++half) {
-                    // W = A X, then the second half of W = X W (A and X are symmetric)
+                    // scratch = A X, then its second half = X scratch (A and X are symmetric)
                     for (int u = blockIdx.x; u < T * T; u += gridDim.x) {
                         const int i = u % T, j = u / T;
                         double acc[4][4];
                         if (half == 0) sym_product_tile(acc, e.A, n, e.out, e.ldo, n, i, j, smem);
-                        else sym_product_tile(acc, e.out, e.ldo, e.W, n, n, i, j, smem);
-                        double* C = half == 0 ? e.W : e.W + (size_t)n * n;
+                        else sym_product_tile(acc, e.out, e.ldo, scratch, n, n, i, j, smem);
+                        double* C = half == 0 ? scratch : scratch + (size_t)n * n;
 #pragma unroll
                         for (int nb = 0; nb < 4; ++nb)
 #pragma unroll
@@ -244,7 +244,7 @@ sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, Source 
                     alive = sym_grid_barrier(barrier, turn);
                 }
                 if (!alive) break;
-                const double* Z = e.W + (size_t)n * n;
+                const double* Z = scratch + (size_t)n * n;
                 double ch = 0.0;                    // largest change over the smaller of its two tile rows' maxima
                 for (long u = blockIdx.x * (long)SYM_THREADS + tid; u < (long)n * n; u += (long)gridDim.x * SYM_THREADS) {
                     const int r = (int)(u % n), c = (int)(u / n);
@@ -288,7 +288,8 @@ sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, Source 
 }
 
 template <class Source>
-int sym_rescue_launch(const SymEntry* entries_dev, int count, unsigned* barrier, Source source, cudaStream_t stream) {
+int sym_rescue_launch(const SymEntry* entries_dev, int count, unsigned* barrier, double* scratch, Source source,
+                      cudaStream_t stream) {
     if (count <= 0) return SCATT_OK;
     int dev = 0, sms = 0;
     SCATT_CUDA_TRY(cudaGetDevice(&dev));
@@ -311,12 +312,12 @@ int sym_rescue_launch(const SymEntry* entries_dev, int count, unsigned* barrier,
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    SCATT_CUDA_TRY(cudaLaunchKernelEx(&cfg, sym_rescue_kernel<Source>, entries_dev, count, barrier, source));
+    SCATT_CUDA_TRY(cudaLaunchKernelEx(&cfg, sym_rescue_kernel<Source>, entries_dev, count, barrier, scratch, source));
     SCATT_COUNT_LAUNCH(1);
     return SCATT_OK;
 }
 
-// For callers whose entry.A is intact; barrier: one zeroed word.
-int sym_rescue_batched(const SymEntry* entries_dev, int count, unsigned* barrier, cudaStream_t stream);
+// For callers whose entry.A is intact; barrier: one zeroed word; scratch: sym_scratch_doubles of the largest order.
+int sym_rescue_batched(const SymEntry* entries_dev, int count, unsigned* barrier, double* scratch, cudaStream_t stream);
 
 }  // namespace scatt

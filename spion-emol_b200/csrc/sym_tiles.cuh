@@ -24,7 +24,7 @@ constexpr int SYM_THREADS = 256;
 // One matrix of a batched symmetric inverse (a device array of these).
 struct SymEntry {
     double* A;              // n x n, ld n (both triangles): rebuilt or kept for the rescue, then its scratch
-    double* W;              // T (T + 1) / 2 tiles, and two n x n matrices for the rescue
+    double* W;              // T (T + 1) / 2 tiles
     double *P, *M;          // T tiles each: the pivot column block and its negated product with D
     double* D;              // the inverse of the pivot tile, the pivot tile itself, and sym_skew of the two
     double* out;            // n x n, ld ldo: the inverse, both triangles
@@ -38,10 +38,12 @@ __host__ __device__ inline int sym_tiles_of(int n) { return (n + SYM_NB - 1) / S
 __host__ __device__ inline size_t sym_tile_index(int i, int j) { return (size_t)i * (i + 1) / 2 + j; }
 // Doubles that W needs for order n, and those of P, M and D together (D: two tiles and a word).
 inline size_t sym_work_doubles(int n) {
-    const size_t T = sym_tiles_of(n), w = T * (T + 1) / 2 * SYM_TILE, full = 2 * (size_t)n * n;
-    return w > full ? w : full;
+    const size_t T = sym_tiles_of(n);
+    return T * (T + 1) / 2 * SYM_TILE;
 }
 inline size_t sym_panel_doubles(int n) { return (2 * (size_t)sym_tiles_of(n) + 2) * SYM_TILE + 32; }
+// Doubles of the rescue's scratch, one for all entries of a batch (it takes one at a time).
+inline size_t sym_scratch_doubles(int n) { return 2 * (size_t)n * n; }
 
 __device__ __forceinline__ int sym_pos(int r, int c) {
     return (((r >> 3) << 3) + (c >> 3)) * 64 + ((r & 7) << 3) + (c & 7);

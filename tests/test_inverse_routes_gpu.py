@@ -44,3 +44,19 @@ def test_the_gradients_forward_is_the_general_solve(l_cont, n_orb):
         for f in FIELDS:
             x, y = getattr(a, f), getattr(b, f)
             assert np.max(np.abs(x - y)) <= 1e-10 * np.max(np.abs(y)), f
+
+
+def test_device_memory_of_a_slot():
+    """A slot of the scan at l_cont 20, N_t 1046 (a group of its own): 158 MB,
+    none of it for the rescue's products, which the slots share."""
+    import torch
+
+    sol = S.ScanSolver(synth.h2o_like(Nr=131, dr=1.4 / 130, l_cont=20, lmax_orb=40, n_orb=5))
+    opts = S.default_opts(allow_closed_channels=1, keep_window=0)
+    used = []
+    for slots in (16, 48):
+        before = torch.cuda.mem_get_info()[0]
+        scan = sol.scan(slots=slots, groups=slots, opts=opts)
+        used.append(before - torch.cuda.mem_get_info()[0])
+        scan.close()
+    assert (used[1] - used[0]) / 32 <= 160e6

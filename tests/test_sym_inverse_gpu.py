@@ -216,3 +216,19 @@ def test_pivots_outside_the_reciprocal(value, at):
     want = np.eye(130)
     want[at, at] = 1.0 / value                      # a subnormal number for the last two
     assert np.all(np.abs(X[0] - want) <= np.where(want == 1.0 / value, np.spacing(want), 0.0))
+
+
+def test_rescued_entries_share_their_scratch():
+    """One, two and no Newton steps and eliminations side by side in a batch."""
+    n, want = 200, [1, 2, 0, 1, 3, 2, 1, 0, 2, 3]
+    A = symmetric(np.random.default_rng(21), len(want), n)
+    for a, m in zip(A, want):
+        if m:
+            a[:64, :64] = {1: 2e-3, 2: 1e-5, 3: 0.0}[m] * np.eye(64)
+            a[:64, 64:128] = a[64:128, :64] = np.eye(64)
+            a[:64, 128:] = a[128:, :64] = 0.0
+    X, st, mode = _lib.inverse_symmetric_batched(A)
+    assert np.all(st == 0) and np.array_equal(mode, want)
+    for a, x in zip(A, X):
+        ref = np.linalg.inv(a)
+        assert np.max(np.abs(x - ref)) <= 1e-13 * max(10.0, np.linalg.cond(a)) * np.max(np.abs(ref))
