@@ -206,7 +206,7 @@ int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* o
         set_last_error("scatt_inverse_symmetric_batched: bad arguments");
         return SCATT_ERR_ARG;
     }
-    if (n > 8192 || count > 65535) {
+    if (n > SYM_ORDER_MAX || count > 65535) {
         set_last_error("scatt_inverse_symmetric_batched: order above 8192 or more than 65535 matrices");
         return SCATT_ERR_SIZE;
     }

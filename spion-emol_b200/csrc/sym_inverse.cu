@@ -374,6 +374,10 @@ int sym_sweep_batched(const SymEntry* entries_dev, int count, int nmax, cudaStre
         set_last_error("sym_sweep_batched: batch count exceeds 65535");
         return SCATT_ERR_ARG;
     }
+    if (nmax > SYM_ORDER_MAX) {
+        set_last_error("sym_sweep_batched: order " + std::to_string(nmax) + " exceeds " + std::to_string(SYM_ORDER_MAX));
+        return SCATT_ERR_SIZE;
+    }
     static std::atomic<unsigned long long> panel_done{0}, update_done{0};
     SCATT_TRY(sym_allow_smem(sym_panel_kernel, PANEL_SMEM, panel_done));
     SCATT_TRY(sym_allow_smem(sym_update_kernel, UPDATE_SMEM, update_done));

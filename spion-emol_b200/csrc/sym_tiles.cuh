@@ -20,6 +20,7 @@ namespace scatt {
 constexpr int SYM_NB = 64;                   // tile order
 constexpr int SYM_TILE = SYM_NB * SYM_NB;    // doubles of a tile
 constexpr int SYM_THREADS = 256;
+constexpr int SYM_ORDER_MAX = 8192;          // the general inverse's limit too
 
 // One matrix of a batched symmetric inverse (a device array of these).
 struct SymEntry {

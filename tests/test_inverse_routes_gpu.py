@@ -60,3 +60,11 @@ def test_device_memory_of_a_slot():
         used.append(before - torch.cuda.mem_get_info()[0])
         scan.close()
     assert (used[1] - used[0]) / 32 <= 160e6
+
+
+def test_orders_above_8192_are_refused():
+    """N_t 8273 (64 orbitals at l_cont 22): an order that neither inverse takes."""
+    sol = S.ScanSolver(synth.h2o_like(Nr=131, dr=1.4 / 130, l_cont=22, lmax_orb=2, n_orb=64))
+    with pytest.raises(_lib.ScattError) as e:
+        sol.solve([0.9], opts=S.default_opts(**OPTS, keep_window=0))
+    assert e.value.code == 3                        # SCATT_ERR_SIZE
