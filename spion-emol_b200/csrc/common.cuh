@@ -75,6 +75,20 @@ __device__ __forceinline__ void dep_sync() {
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
+// Once per device: the most dynamic shared memory that any launch of `kernel`
+// takes (a kernel's attribute is the process's: set to one call's size, another
+// thread's smaller call could lower it before this one's launch).  `done` has a
+// bit per device.
+template <class... P>
+int allow_smem(void (*kernel)(P...), size_t bytes, std::atomic<unsigned long long>& done) {
+    int dev = 0;
+    SCATT_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && (done.load() & (1ull << dev))) return SCATT_OK;
+    SCATT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (dev >= 0 && dev < 64) done.fetch_or(1ull << dev);
+    return SCATT_OK;
+}
+
 // Device-side status codes written into per-matrix status words.
 enum DeviceStatus : int {
     DEV_OK = 0,

@@ -196,15 +196,17 @@ bisect_kernel(const EigEntry* entries, int nwant) {
 int sym_eigvals_batched(const EigEntry* entries_dev, int count, int nmax, int nwant,
                         cudaStream_t stream) {
     if (count <= 0 || nmax <= 0) return SCATT_OK;
-    const size_t ts = 3 * (size_t)nmax * sizeof(double), bs = 2 * (size_t)nmax * sizeof(double);
-    if (ts > 200 * 1024) {
+    // orders of S(n) and K, whose inverses end at 8192
+    constexpr size_t order_max = 8533;
+    static_assert(3 * order_max * sizeof(double) <= 200 * 1024, "one CTA's shared memory");
+    if ((size_t)nmax > order_max) {
         set_last_error("sym_eigvals_batched: order above 8533");
         return SCATT_ERR_SIZE;
     }
-    if (ts > 48 * 1024)
-        SCATT_CUDA_TRY(cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts));
-    if (bs > 48 * 1024)
-        SCATT_CUDA_TRY(cudaFuncSetAttribute(bisect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bs));
+    static std::atomic<unsigned long long> tridiag_done{0}, bisect_done{0};
+    SCATT_TRY(allow_smem(tridiag_kernel, 3 * order_max * sizeof(double), tridiag_done));
+    SCATT_TRY(allow_smem(bisect_kernel, 2 * order_max * sizeof(double), bisect_done));
+    const size_t ts = 3 * (size_t)nmax * sizeof(double), bs = 2 * (size_t)nmax * sizeof(double);
     tridiag_kernel<<<count * EC, ET, ts, stream>>>(entries_dev);
     const int want = nwant > 0 ? nwant : nmax;
     bisect_kernel<<<dim3((want + BT - 1) / BT, count), BT, bs, stream>>>(entries_dev, nwant);

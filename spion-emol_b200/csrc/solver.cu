@@ -1882,7 +1882,7 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                 if (sym_r) {
                     const int T = sym_tiles_of(sc.Nt_cap), nt = T * (T + 1) / 2;
                     static std::atomic<unsigned long long> done{0};
-                    SCATT_TRY(sym_allow_smem(k_assemble_R_tiles, sizeof(SymDiagShared), done));
+                    SCATT_TRY(allow_smem(k_assemble_R_tiles, sizeof(SymDiagShared), done));
                     SCATT_TRY(run(k_assemble_R_tiles, dim3(count * nt), SYM_THREADS, sizeof(SymDiagShared), b, j, nt));
                 }
                 if (gen_r) SCATT_TRY(run(k_assemble_R, eg, TPB, 0, b, j));

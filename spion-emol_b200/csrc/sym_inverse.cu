@@ -362,7 +362,7 @@ int sym_pack_batched(const SymEntry* entries_dev, int count, int nmax, cudaStrea
     const int T = sym_tiles_of(nmax);
     const int nt = T * (T + 1) / 2;
     static std::atomic<unsigned long long> done{0};
-    SCATT_TRY(sym_allow_smem(sym_pack_kernel, sizeof(SymDiagShared), done));
+    SCATT_TRY(allow_smem(sym_pack_kernel, sizeof(SymDiagShared), done));
     SCATT_CUDA_TRY(launch_dep(sym_pack_kernel, count * nt, SYM_THREADS, sizeof(SymDiagShared), stream, entries_dev, count, nt));
     SCATT_COUNT_LAUNCH(1);
     return SCATT_OK;
@@ -379,8 +379,8 @@ int sym_sweep_batched(const SymEntry* entries_dev, int count, int nmax, cudaStre
         return SCATT_ERR_SIZE;
     }
     static std::atomic<unsigned long long> panel_done{0}, update_done{0};
-    SCATT_TRY(sym_allow_smem(sym_panel_kernel, PANEL_SMEM, panel_done));
-    SCATT_TRY(sym_allow_smem(sym_update_kernel, UPDATE_SMEM, update_done));
+    SCATT_TRY(allow_smem(sym_panel_kernel, PANEL_SMEM, panel_done));
+    SCATT_TRY(allow_smem(sym_update_kernel, UPDATE_SMEM, update_done));
     const int T = sym_tiles_of(nmax), nu = T * (T - 1) / 2;
     for (int K = 0; K < T; ++K) {
         SCATT_CUDA_TRY(launch_dep(sym_panel_kernel, dim3(2 * T, count), SYM_THREADS, PANEL_SMEM, stream, entries_dev, K));

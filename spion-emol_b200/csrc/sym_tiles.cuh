@@ -448,15 +448,4 @@ int sym_sweep_batched(const SymEntry* entries_dev, int count, int nmax, cudaStre
 // Packs full symmetric matrices (entry.A) for sym_sweep_batched; stat and status must be zero.
 int sym_pack_batched(const SymEntry* entries_dev, int count, int nmax, cudaStream_t stream);
 
-// Once per device: the dynamic shared memory that `kernel` may ask for; `done` has a bit per device.
-template <class... P>
-int sym_allow_smem(void (*kernel)(P...), size_t bytes, std::atomic<unsigned long long>& done) {
-    int dev = 0;
-    SCATT_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64 && (done.load() & (1ull << dev))) return SCATT_OK;
-    SCATT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    if (dev >= 0 && dev < 64) done.fetch_or(1ull << dev);
-    return SCATT_OK;
-}
-
 }  // namespace scatt
