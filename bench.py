@@ -2,7 +2,7 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
                     [--config h2o_like|h2_like|h2o_mixed|c8f8_like] [--slots S] [--groups G]
-                    [--graphs 0|1] [--autotune 0|1]
+                    [--graphs 0|1]
 
 Workload (default): the H2O-like system -- O + 2 H, five doubly occupied
 orbitals, l_cont = 20 (441 continuum + 605 exchange channels, N_t = 1046),
@@ -102,7 +102,7 @@ def predict_seconds(config: str, slots: int, groups: int, steps: int, warmup: in
                     cpu_s: float = 30.0) -> float:
     """Wall time of `bench.py --config C --steps K --warmup W`: the chunks at
     the measured cost per chunk (post stages included in it), plus setup
-    (upload, cuBLAS peak, autotune) and the CPU baseline."""
+    (upload, cuBLAS peak) and the CPU baseline."""
     fixed, per_slot = CHUNK_S[config]
     return setup_s + cpu_s + plan(config, slots, groups, steps, warmup)["chunks_total"] * (fixed + per_slot * slots)
 
@@ -307,8 +307,6 @@ def main():
     ap.add_argument("--graphs", type=int, default=-1, help="replay chunks from CUDA graphs (default: per config)")
     ap.add_argument("--keep-window", type=int, default=0,
                     help="1: keep the fit window store (fit residual diagnostics); 0: accumulate the fit forward")
-    ap.add_argument("--autotune", type=int, default=1,
-                    help="time the inverse's blockings for the workload's orders before the run")
     ap.add_argument("--cpu-budget", type=float, default=20.0,
                     help="seconds of oracle work per CPU sample (the reference arm takes one per step)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
@@ -352,7 +350,6 @@ def main():
                                 timeout=__import__("datetime").timedelta(seconds=600))
     torch.cuda.set_device(local)
     from scatt_b200 import solver as S
-    from scatt_b200 import _lib
 
     inp = getattr(synth, cfg["builder"])(**cfg["kw"])
     t0 = time.time()
@@ -371,14 +368,6 @@ def main():
         cursor[0] += n
         return Es_all[idx], lc_mine[idx]
 
-    tuned = []
-    if a.autotune:
-        # inverses of the scan's batches: R^-1 of order N_t over the slots, and the
-        # Schur inverses of order Np over the slots' 8 radial steps of a chunk
-        # (orders above 1280 have one blocking, the cluster panel: nothing to tune)
-        for n, count in sorted({(sol.Np + sol.Nf, slots), (sol.Np, slots * 8)}):
-            if n <= 1280:
-                tuned.append(_lib.autotune_inverse(n, count, device=local))
     peak = cuda_dgemm_peak(torch) if rank == 0 else None
     alloc, _keep = pinned_alloc(torch)
     opts = S.default_opts(allow_closed_channels=1, timing=1, use_graphs=graphs, keep_window=a.keep_window)
@@ -431,7 +420,7 @@ def main():
             "config": {**workload, "parallelism": f"energy-sharded x{ws}", "cuda_graphs": bool(graphs),
                        "fit": "window store and back sweep (fit residual diagnostics)" if a.keep_window else
                               "accumulated forward, [A; B] = G_A(N-1)^T Z_N (no window store; fit residual not computed)",
-                       "autotuned_inverses": tuned,
+                       "inverse": "S and R by the symmetric sweep on 64 x 64 tiles (nothing to tune)",
                        "l2": "inputs larger than L2 (the scan's device state, several GB, exceeds the 126 MB L2)"},
             "e2e": {"value": n_total / host_s, "unit": "energies/s", "h2d_bytes_per_step": 8 * gsize,
                     "d2h_bytes_per_step": int(out_bytes / max(a.steps, 1))},
