@@ -243,7 +243,7 @@ __device__ __forceinline__ SymEntry sym_entry(double* A, double* W, double* pane
 // that the chunk changes).  Entries of steps outside a slot's chunk, and of
 // stages a step does not take, are empty (M = 0, n = 0): the kernels skip them.
 // An inverse has one of its two entries filled: with `symmetric` the sweep's
-// where the slot's own order is above one tile, else the general inverse's.
+// where the slot's own N_t is above one tile, else the general inverse's.
 __global__ void k_prepare(BatchDev b, bool symmetric) {
     dep_sync();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -278,10 +278,10 @@ __global__ void k_prepare(BatchDev b, bool symmetric) {
     const double* Cn = (n < b.n_pts) ? b.Ctab + (size_t)n * K * b.Np_max : nullptr;
     // Bs B^T = B D^-1 B^T and A are symmetric: lower tiles only, mirrored
     b.gmS[idx] = exch ? GemmEntry{Bs, B_of(b, d, j), S, Np, Np, Nf, b.Np_max, b.Np_max, Np, -1.0, 1.0, 1} : none;
-    const bool symS = symmetric && Np > SYM_NB, symR = symmetric && Nt > SYM_NB;
+    const bool sym = symmetric && Nt > SYM_NB;
     b.gjS[idx] = GjEntry{S, d.Sw + j * b.sw_stride, sinv, d.sigS + (size_t)j * Np, d.ridS + (size_t)j * Np,
-                         d.stS + 4 * j, symS ? 0 : Np, Np, Np, d.PS + j * b.ps_stride, d.sgS + (size_t)j * 4 * Np};
-    if (symS) b.syS[idx] = sym_entry(S, d.Sw + j * b.sw_stride, d.PS + j * b.ps_stride, sinv,
+                         d.stS + 4 * j, sym ? 0 : Np, Np, Np, d.PS + j * b.ps_stride, d.sgS + (size_t)j * 4 * Np};
+    if (sym) b.syS[idx] = sym_entry(S, d.Sw + j * b.sw_stride, d.PS + j * b.ps_stride, sinv,
                                      b.stat + ((size_t)b.count * SCHUR_CHUNK + idx) * b.stat_stride, d.stS + 4 * j, Np);
     else b.syS[idx].n = 0;
     b.gmT[idx] = exch ? GemmEntry{sinv, Bs, d.T, Np, Nf, Np, Np, b.Np_max, Np, 1.0, 0.0} : none;
@@ -296,9 +296,9 @@ __global__ void k_prepare(BatchDev b, bool symmetric) {
                                   2 * Np, 1.0, 0.0}
                       : none;
     const bool inv = n >= b.n_start;
-    b.gjR[idx] = GjEntry{d.Ra, d.Rw, rinv, d.sigR, d.ridR, d.stR + 4 * j, inv && !symR ? Nt : 0, Nt, Nt, d.PR, d.sgR};
+    b.gjR[idx] = GjEntry{d.Ra, d.Rw, rinv, d.sigR, d.ridR, d.stR + 4 * j, inv && !sym ? Nt : 0, Nt, Nt, d.PR, d.sgR};
     if (inv) b.rargs[idx] = RArgs{sinv, d.T, d.F, Dinv_of(b, d, j), rinv_at(b, d, n - 1), Np, Nt, Nf, n < b.n_tr};
-    if (inv && symR) b.syR[idx] = sym_entry(d.Ra, d.Rw, d.PR, rinv, b.stat + (size_t)idx * b.stat_stride,
+    if (inv && sym) b.syR[idx] = sym_entry(d.Ra, d.Rw, d.PR, rinv, b.stat + (size_t)idx * b.stat_stride,
                                              d.stR + 4 * j, Nt);
     else b.syR[idx].n = 0;
 }
@@ -1423,11 +1423,12 @@ int ensure_stab(Context& ctx, const scatt_solve_opts& o, int l_cont, const doubl
 
 // Doubles of the panel buffers of one inverse of order n: the Gauss-Jordan
 // windows (four, with the look-ahead) or the symmetric sweep's P, M and D.
-size_t panel_doubles(int n) {
-    return std::max((size_t)4 * GJ_WINDOW_MAX * n, n > SYM_NB ? sym_panel_doubles(n) : 0);
+// (in slots that may take it, N_t above one tile).
+size_t panel_doubles(int n, int Nt) {
+    return std::max((size_t)4 * GJ_WINDOW_MAX * n, Nt > SYM_NB ? sym_panel_doubles(n) : 0);
 }
 // Doubles of its work buffer: n x n for the Gauss-Jordan, or the sweep's tiles.
-size_t work_doubles(int n) { return std::max((size_t)n * n, n > SYM_NB ? sym_work_doubles(n) : 0); }
+size_t work_doubles(int n, int Nt) { return std::max((size_t)n * n, Nt > SYM_NB ? sym_work_doubles(n) : 0); }
 
 // Device doubles of one slot sized for (Np, Nt): the chunk's Schur slots,
 // the W^-1 blocks, the R ping-pong buffers, the dipole rows, the asymptotic
@@ -1439,9 +1440,10 @@ size_t slot_doubles(const BatchDev& b, int Np, int Nt, int l_cont, bool keep_win
     const int nslots = b.N - b.n_s + 1;
     auto al = [](size_t c) { return (c + 31) & ~size_t(31); };
     const size_t np2 = (size_t)Np * Np, nt2 = (size_t)Nt * Nt;
-    const size_t base = 2 * al(SCHUR_CHUNK * np2) + al(SCHUR_CHUNK * al(work_doubles(Np))) +
-                        al((size_t)Np * b.Nf) + al((size_t)b.Nf * b.Nf) + 3 * al(nt2) + al(work_doubles(Nt)) +
-                        2 * al((size_t)b.Krows * Nt) + al(SCHUR_CHUNK * al(panel_doubles(Np))) + al(panel_doubles(Nt));
+    const size_t base = 2 * al(SCHUR_CHUNK * np2) + al(SCHUR_CHUNK * al(work_doubles(Np, Nt))) +
+                        al((size_t)Np * b.Nf) + al((size_t)b.Nf * b.Nf) + 3 * al(nt2) + al(work_doubles(Nt, Nt)) +
+                        2 * al((size_t)b.Krows * Nt) + al(SCHUR_CHUNK * al(panel_doubles(Np, Nt))) +
+                        al(panel_doubles(Nt, Nt));
     if (keep_window) return base + al((size_t)nslots * nt2) + 2 * al((size_t)nslots * np2);
     return base + 2 * al((size_t)2 * Np * Nt) + al((size_t)b.nfit * 2 * Np) + al((size_t)8 * (l_cont + 1));
 }
@@ -1596,8 +1598,8 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
     sc.nfit = sc.ne_fit - b.n_s + 1;
     b.count = slots;
     b.ngroups = ngroups;
-    b.sw_stride = (work_doubles(sc.Np_cap) + 31) & ~size_t(31);
-    b.ps_stride = (panel_doubles(sc.Np_cap) + 31) & ~size_t(31);
+    b.sw_stride = (work_doubles(sc.Np_cap, sc.Nt_cap) + 31) & ~size_t(31);
+    b.ps_stride = (panel_doubles(sc.Np_cap, sc.Nt_cap) + 31) & ~size_t(31);
     const int K = b.Krows, Nf = b.Nf;
     // ---- slot arena
     const bool keep = o.keep_window != 0;
@@ -1621,7 +1623,7 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
         d.T = take((size_t)sc.Np_cap * Nf);
         d.F = take((size_t)Nf * Nf);
         d.Ra = take(nt2);
-        d.Rw = take(work_doubles(sc.Nt_cap));
+        d.Rw = take(work_doubles(sc.Nt_cap, sc.Nt_cap));
         d.Rinv0 = take(nt2);
         d.Rinv1 = take(nt2);
         d.G0 = take((size_t)K * sc.Nt_cap);
@@ -1637,7 +1639,7 @@ int scan_open(Context& ctx, const scatt_solve_opts& o, int slots, int ngroups, i
             d.Mab = take((size_t)8 * (l_cap + 1));
         }
         d.PS = take(SCHUR_CHUNK * b.ps_stride);
-        d.PR = take(panel_doubles(sc.Nt_cap));
+        d.PR = take(panel_doubles(sc.Nt_cap, sc.Nt_cap));
         int* q = sc.iarena.p + slot_ints(sc.Np_cap, sc.Nt_cap) * e;
         const int Np = sc.Np_cap, Nt = sc.Nt_cap;
         d.sigS = q; q += SCHUR_CHUNK * Np;
@@ -1809,15 +1811,15 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
     // S and R are symmetric: the automatic scheme takes the symmetric sweep (half the flops, no
     // column of pivots); the forced schemes keep the general inverse
     const bool symmetric = !sc.general && g_inverse_scheme.load(std::memory_order_relaxed) == 0;
-    // Orders of one tile stay with the general inverse, slot by slot: the sweep would be one pivot
-    // chain, no faster, and its eight-column panels leave a few times the rounding of the general
-    // inverse's sixteen (an objective's noise at N_t 64: 1.0e-14 against 1.0e-15)
-    bool gen_s = false, sym_s = false, gen_r = false, sym_r = false;     // what the running slots need
+    // Slots whose R is one tile stay with the general inverse: the sweep would be one pivot chain, no
+    // faster, and its eight-column panels leave a few times the rounding of the general inverse's
+    // sixteen (an objective's noise at N_t 64: 1.0e-14 against 1.0e-15).  That is not so of S, near
+    // the unit matrix (orders 16 and 49: errors within 5 % of each other), which goes with its R:
+    // the general inverse of S of order 49 takes 60 us a chunk longer.
+    bool gen = false, sweeps = false;                                    // what the running slots need
     for (int e = 0; e < count; ++e) {
         const EnergyDev& d = sc.ed[e];
-        if (!d.live || sc.grp[d.grp].n0 < 0) continue;
-        (symmetric && d.Np > SYM_NB ? sym_s : gen_s) = true;
-        (symmetric && d.Nt > SYM_NB ? sym_r : gen_r) = true;
+        if (d.live && sc.grp[d.grp].n0 >= 0) (symmetric && d.Nt > SYM_NB ? sweeps : gen) = true;
     }
     const int gen_Np = symmetric ? std::min(sc.Np_cap, SYM_NB) : sc.Np_cap;
     const int gen_Nt = symmetric ? std::min(sc.Nt_cap, SYM_NB) : sc.Nt_cap;
@@ -1858,12 +1860,12 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
         SCATT_TRY(run(k_prepare, dim3(cdiv(count * SCHUR_CHUNK, 128)), 128, 0, b, symmetric));
         if (any_exch) SCATT_TRY(gemm_slots(sc, b.gmS, count * SCHUR_CHUNK, 0, 0, 1));
         if (stab_x) SCATT_TRY(run(k_stab, dim3(count, SCHUR_CHUNK), TPB, 0, b, 1));
-        if (sym_s) {
+        if (sweeps) {
             SCATT_TRY(sym_pack_batched(b.syS, count * SCHUR_CHUNK, sc.Np_cap, s));
             SCATT_TRY(sym_sweep_batched(b.syS, count * SCHUR_CHUNK, sc.Np_cap, s));
             SCATT_TRY(sym_rescue_batched(b.syS, count * SCHUR_CHUNK, b.barrier + SCHUR_CHUNK, sc.scratch.p, s));
         }
-        if (gen_s) SCATT_TRY(gj_inverse_selected(b.gjS, count * SCHUR_CHUNK, gen_Np, true, s, true));
+        if (gen) SCATT_TRY(gj_inverse_selected(b.gjS, count * SCHUR_CHUNK, gen_Np, true, s, true));
         // ---- the R-ratio recurrence over the chunk's steps
         const dim3 eg(64, count);
         for (int j = 0; j < SCHUR_CHUNK; ++j) {
@@ -1879,13 +1881,13 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                 SCATT_TRY(run(k_analytic_R_diag, dim3(4, count), TPB, 0, b, j));
             }
             if (rinv[j]) {
-                if (sym_r) {
+                if (sweeps) {
                     const int T = sym_tiles_of(sc.Nt_cap), nt = T * (T + 1) / 2;
                     static std::atomic<unsigned long long> done{0};
                     SCATT_TRY(allow_smem(k_assemble_R_tiles, sizeof(SymDiagShared), done));
                     SCATT_TRY(run(k_assemble_R_tiles, dim3(count * nt), SYM_THREADS, sizeof(SymDiagShared), b, j, nt));
                 }
-                if (gen_r) SCATT_TRY(run(k_assemble_R, eg, TPB, 0, b, j));
+                if (gen) SCATT_TRY(run(k_assemble_R, eg, TPB, 0, b, j));
                 const bool sample = sample_chunk && j == 0;
                 cudaEvent_t a0 = nullptr, a1 = nullptr;
                 if (sample) {
@@ -1893,11 +1895,11 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
                     SCATT_TRY(sc.events.get(&a1));
                     SCATT_CUDA_TRY(cudaEventRecord(a0, s));
                 }
-                if (sym_r) {
+                if (sweeps) {
                     SCATT_TRY(sym_sweep_batched(b.syR + at, count, sc.Nt_cap, s));
                     SCATT_TRY(sym_rescue_launch(b.syR + at, count, b.barrier + j, sc.scratch.p, RSource{b, j}, s));
                 }
-                if (gen_r) SCATT_TRY(gj_inverse_selected(b.gjR + at, count, gen_Nt, true, s, true));
+                if (gen) SCATT_TRY(gj_inverse_selected(b.gjR + at, count, gen_Nt, true, s, true));
                 if (sample) {
                     SCATT_CUDA_TRY(cudaEventRecord(a1, s));
                     tm->rinv.push_back({a0, a1});
@@ -1923,9 +1925,8 @@ int run_chunk(Scan& sc, ChunkTiming* tm) {
         SCATT_TRY(run(k_advance, dim3(1), MAX_GROUPS, 0, b));
         return SCATT_CUDA_TRY_RET(cudaGetLastError());
     };
-    uint64_t key = (stab ? 1u : 0u) | (stab_x ? 2u : 0u) | (any_exch ? 4u : 0u) | ((uint64_t)gen_s << 59) |
-                   ((uint64_t)sym_s << 60) | ((uint64_t)gen_r << 61) | ((uint64_t)sym_r << 62) |
-                   ((uint64_t)symmetric << 63);
+    uint64_t key = (stab ? 1u : 0u) | (stab_x ? 2u : 0u) | (any_exch ? 4u : 0u) | ((uint64_t)gen << 59) |
+                   ((uint64_t)sweeps << 60) | ((uint64_t)symmetric << 61);
     for (int j = 0; j < SCHUR_CHUNK; ++j) {
         const uint64_t bits = (step[j] ? 1u : 0u) | (exch[j] ? 2u : 0u) | (start[j] ? 4u : 0u) |
                               (rinv[j] ? 8u : 0u) | (sweep[j] ? 16u : 0u) | (pts[j] ? 32u : 0u) |

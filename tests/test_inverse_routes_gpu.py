@@ -1,6 +1,6 @@
-"""Which inverse the solver takes for S(n) and R(n): orders of one 64 x 64 tile
-the general one, also beside the symmetric sweep of the others; the gradients
-the general one throughout."""
+"""Which inverse the solver takes for S(n) and R(n): the general one where R is
+one 64 x 64 tile (N_t <= 64), the symmetric sweep above; the gradients the
+general one throughout."""
 import numpy as np
 import pytest
 
