@@ -232,3 +232,37 @@ def test_rescued_entries_share_their_scratch():
     for a, x in zip(A, X):
         ref = np.linalg.inv(a)
         assert np.max(np.abs(x - ref)) <= 1e-13 * max(10.0, np.linalg.cond(a)) * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("n", [2049, 5317, 8192])
+def test_large_orders(n):
+    """Up to the largest order accepted, by the residual on a few vectors
+    (kappa as in the family above: rounding of n-term sums)."""
+    rng = np.random.default_rng(n)
+    M = rng.standard_normal((n, n))
+    M += M.T.copy()
+    M *= 0.9 / (2.0 * np.sqrt(2.0 * n))
+    i = np.arange(n)
+    M[i, i] += np.where(i % 5 == 0, -2.0, 2.0)
+    X, st, mode = _lib.inverse_symmetric_batched(M[None])
+    assert st[0, 0] == 0 and mode[0] == 0
+    x = rng.standard_normal((n, 3))
+    assert np.linalg.norm(X[0] @ (M @ x) - x) <= 1e-13 * np.linalg.norm(x)
+    assert np.linalg.norm(X[0].T @ x - X[0] @ x) <= 1e-14 * np.linalg.norm(X[0] @ x)
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("at", [(0, 0), (70, 3), (99, 99)])
+def test_nonfinite_elements(value, at):
+    A = symmetric(np.random.default_rng(2), 3, 100)
+    A[1, at[0], at[1]] = A[1, at[1], at[0]] = value
+    X, st, _ = _lib.inverse_symmetric_batched(A)
+    assert list(st[:, 0]) == [0, 2, 0]
+    for b in (0, 2):
+        ref = np.linalg.inv(A[b])
+        assert np.max(np.abs(X[b] - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+def test_orders_and_batches_refused():
+    with pytest.raises(_lib.ScattError):
+        _lib.inverse_symmetric_batched(np.zeros((1, 8193, 8193)))
