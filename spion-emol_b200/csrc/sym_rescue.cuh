@@ -13,7 +13,11 @@
 // rarer the finer the grid), and a second one above g = 1e3.  Not elsewhere: the step leaves rounding of
 // kappa eps, which a sweep of a graded matrix (large diagonal elements near
 // the origin) stays ten times below.  What a badly conditioned pivot tile does
-// without growth is met in the sweep itself (SYM_SKEW_MAX).
+// without growth is met in the sweep itself (SYM_SKEW_MAX); above a skew of 1e3
+// (1 in 85 matrices of a sweep at 0.05 bohr, order 1046) a step follows there
+// too: it halves the inverse's error on average, and where the next R is nearly
+// singular the error that reaches its inverse fell from 2.1e-11 to 5.1e-12
+// (the general inverse: 2.7e-12).
 // Measured on the matrices of one sweep (order 1046, kappa = max|A| max|X|),
 // relative errors:
 //              g       kappa   sweep    Newton   LU       Gauss-Jordan, pivoted
@@ -30,6 +34,9 @@
 #include "sym_tiles.cuh"
 
 namespace scatt {
+
+// Largest sym_skew that the refined rows (sym_panel_kernel) are left with.
+constexpr double SYM_SKEW_NEWTON = 1e3;
 
 // Barrier over the grid's CTAs, all resident (cooperative launch): `turn`
 // counts the barriers passed on this counter, which starts at zero.  The wait
@@ -204,9 +211,10 @@ sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, double*
                 bad |= !isfinite(a) || !isfinite(s) || !isfinite(d) || !isfinite(x) || !(a > 0.0) || !(x > 0.0);
             }
             for (int o = 1; o <= 2; o <<= 1) gr = fmax(gr, __shfl_xor_sync(0xffffffffu, gr, o));
+            const double skew = n > 0 ? __hiloint2double((int)stat[SYM_STAT_SKEW], 0) : 0.0;
             const unsigned quad = __ballot_sync(0xffffffffu, bad) >> (lane & ~3) & 15u;
             // one tile is pivoted throughout
-            const int mode = n == 0 ? 0 : quad || !(gr <= 1e6) ? 3 : n <= SYM_NB ? 0 : gr > 1e3 ? 2 : gr > 3.0 ? 1 : 0;
+            const int mode = n == 0 ? 0 : quad || !(gr <= 1e6) ? 3 : n <= SYM_NB ? 0 : gr > 1e3 ? 2 : gr > 3.0 || skew > SYM_SKEW_NEWTON ? 1 : 0;
             if (k < m && (tid & 3) == 0) {
                 s_mode[k] = mode;
                 if (n > 0 && blockIdx.x == 0) stat[0] = (unsigned)mode;

@@ -30,7 +30,7 @@ struct SymEntry {
     double* D;              // the inverse of the pivot tile, the pivot tile itself, and sym_skew of the two
     double* out;            // n x n, ld ldo: the inverse, both triangles
     unsigned* stat;         // sym_stat_words(n) words, zero before the sweep: [0] how it was finished, [1 ..] SYM_STEPS Newton
-                            // steps' changes, SYM_STAT_HEAD on sym_stat
+                            // steps' changes, [4] the largest sym_skew (high word), SYM_STAT_HEAD on sym_stat
     int* status;            // DeviceStatus, first failing column; zero before the sweep
     int n, ldo;
 };
@@ -78,7 +78,7 @@ __device__ __forceinline__ unsigned sym_hi(double v) { return (unsigned)__double
 // tile row, of that row in any Schur complement, of the pivot tile's inverse
 // D_i, and of the inverse's tile row.
 enum SymStat { SYM_OF_A = 0, SYM_OF_SCHUR = 1, SYM_OF_D = 2, SYM_OF_X = 3 };
-constexpr int SYM_STEPS = 3, SYM_STAT_HEAD = 1 + SYM_STEPS;
+constexpr int SYM_STEPS = 3, SYM_STAT_SKEW = 4, SYM_STAT_HEAD = 8;
 __host__ __device__ inline size_t sym_stat_words(int n) { return SYM_STAT_HEAD + 4 * (size_t)sym_tiles_of(n); }
 __device__ __forceinline__ unsigned* sym_stat(const SymEntry& e, int i, SymStat q) { return e.stat + SYM_STAT_HEAD + 4 * i + q; }
 // A warp's part of an element block of tile (i, j): it counts for both tile rows.
@@ -105,16 +105,16 @@ static_assert(offsetof(SymDiagShared, panel) % 16 == 0 && offsetof(SymDiagShared
               offsetof(SymDiagShared, low) % 16 == 0, "read and written in 16-byte pieces");
 
 // Pivot tiles whose largest column sum of |A_ij D_ij| (A the tile, D its
-// inverse; sym_skew holds the largest of each warp's columns) is above this have their rows L = P D refined (sym_panel_kernel).
-// The sum is 1 for a diagonal or a well-conditioned dominant tile, does not
-// change when rows and columns are scaled alike (a tile graded by its
-// centrifugal terms has a condition number of 1e3 and a sum below 1.4), and
-// grows with the rounding that D brings into L P^T.  Up to 4, sweeps without
-// the refinement stayed within 1.5 of the general inverse's error over the
-// matrices of radial sweeps (orders 162 and 196, 20 and 50 bohr); above, they
-// did not always.  At 1.4 bohr no tile is above 2, at 20 bohr and order 1046
-// one in 50.
-constexpr double SYM_SKEW_MAX = 2.0;
+// inverse; sym_skew holds the largest of each warp's columns) is above this
+// have their rows L = P D refined (sym_panel_kernel).  The sum is 1 for a
+// diagonal or a well-conditioned dominant tile, does not change when rows and
+// columns are scaled alike (a tile graded by its centrifugal terms has a
+// condition number of 1e3 and a sum below 1.4), and grows with the rounding
+// that D brings into L P^T.  Up to 4, sweeps without the refinement stayed
+// within 1.5 of the general inverse's error over the matrices of radial sweeps
+// (orders 162 and 196, 20 and 50 bohr); above, they did not always.  At 1.4
+// bohr no tile is above it; at 20 bohr and order 1046 one in 50.
+constexpr double SYM_SKEW_MAX = 3.0;
 __device__ __forceinline__ double* sym_tile_of_D(const SymEntry& e) { return e.D + SYM_TILE; }
 __device__ __forceinline__ double* sym_skew(const SymEntry& e) { return e.D + 2 * SYM_TILE; }
 
@@ -384,7 +384,10 @@ __device__ __forceinline__ void sym_diag_store(const SymEntry& e, int K, const S
     s0 = fmax(s0, s1);
 #pragma unroll
     for (int o = 2; o >= 1; o >>= 1) s0 = fmax(s0, __shfl_xor_sync(0xffffffffu, s0, o));
-    if (lane == 0) sym_skew(e)[C] = s0;
+    if (lane == 0) {
+        sym_skew(e)[C] = s0;
+        atomicMax(e.stat + SYM_STAT_SKEW, sym_hi(s0));
+    }
 }
 
 // Packs tile t of entry e from elem(row, column, inside) (the element of a
