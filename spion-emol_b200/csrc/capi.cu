@@ -235,7 +235,7 @@ int scatt_inverse_symmetric_batched(int n, int count, const double* A, double* o
     for (int b = 0; b < count; ++b) {
         double* P = dP.p + ps * b;
         ent[b] = SymEntry{dA.p + nn * b, dW.p + ws * b, P, P + T * SYM_TILE, P + 2 * T * SYM_TILE,
-                          dO.p + nn * b, dstat.p + words * b, dst.p + 2 * b, n, n};
+                          dO.p + nn * b, dstat.p + words * b, dst.p + 2 * b, n, n, SYM_SKEW_MAX};
     }
     DevBuf<SymEntry> dent;
     SCATT_TRY(dent.upload(ent));

@@ -149,7 +149,7 @@ sym_panel_kernel(const SymEntry* entries, int K) {
     for (int u = tid; u < SYM_TILE / 2; u += SYM_THREADS) cp16(Ds + 2 * u, e.D + 2 * u);
     cp_commit();
     // read by one warp of the CTA: read by all, 272 warps at order 1046 queue for one line (0.5 us)
-    const bool skewed = tid < SYM_THREADS / 32 && sym_skew(e)[tid] > SYM_SKEW_MAX;
+    const bool skewed = tid < SYM_THREADS / 32 && sym_skew(e)[tid] > e.skew_max;
     cp_wait<0>();
     const bool refine = __syncthreads_or(skewed);
     double acc[2][4];

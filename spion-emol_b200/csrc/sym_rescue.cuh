@@ -12,16 +12,16 @@
 // which squares the relative error, where g > 3 (rare in a radial sweep, and
 // rarer the finer the grid), and a second one above g = 1e3.  Not elsewhere: the step leaves rounding of
 // kappa eps, which a sweep of a graded matrix (large diagonal elements near
-// the origin) stays ten times below.  What a badly conditioned pivot tile does
-// without growth is met in the sweep itself (SYM_SKEW_MAX); above a skew of 1e3
-// (1 in 85 matrices of a sweep at 0.05 bohr, order 1046) a step follows there
-// too: it halves the inverse's error on average, and where the next R is nearly
-// singular the error that reaches its inverse fell from 2.1e-11 to 5.1e-12
-// (the general inverse: 2.7e-12).
+// the origin) stays ten times below.  A step too where max|D| times A's
+// largest element off the diagonal tiles is above 2e4: one dominant direction
+// that every tile has a part of.  (By sym_skew above 1e3 instead, the dipoles of
+// a sweep at l_cont 11, N_t 386, came out ten times worse, 8.4e-10 off the
+// oracle's.)
 // Measured on the matrices of one sweep (order 1046, kappa = max|A| max|X|),
 // relative errors:
 //              g       kappa   sweep    Newton   LU       Gauss-Jordan, pivoted
 //              1200    21      3.9e-11  7.7e-16  8.4e-16  1.1e-14
+//              0.94    2.1e6   3.1e-9   8.2e-13  1.9e-12  2.7e-13
 //              15      1.4e3   7.7e-13  7.0e-15  3.9e-13  7.4e-13
 //   median     1       20      7e-16             6e-16
 // The steps' changes tell whether they converge: a step more is taken while
@@ -34,9 +34,6 @@
 #include "sym_tiles.cuh"
 
 namespace scatt {
-
-// Largest sym_skew that the refined rows (sym_panel_kernel) are left with.
-constexpr double SYM_SKEW_NEWTON = 1e3;
 
 // Barrier over the grid's CTAs, all resident (cooperative launch): `turn`
 // counts the barriers passed on this counter, which starts at zero.  The wait
@@ -200,7 +197,7 @@ sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, double*
         for (int k = tid >> 2; k < ((m + 7) & ~7); k += SYM_THREADS / 4) {
             const int n = k < m ? entries[base + k].n : 0;
             unsigned* stat = entries[base + min(k, m - 1)].stat;
-            double gr = 0.0;
+            double gr = 0.0, dm = 0.0;
             bool bad = false;
 #pragma unroll 5
             for (int i = tid & 3; i < sym_tiles_of(n); i += 4) {
@@ -208,13 +205,17 @@ sym_rescue_kernel(const SymEntry* entries, int count, unsigned* barrier, double*
                 const double a = __hiloint2double((int)w.x, 0), s = __hiloint2double((int)w.y, 0);
                 const double d = __hiloint2double((int)w.z, 0), x = __hiloint2double((int)w.w, 0);
                 gr = fmax(gr, fmax(d / x, s / a));
+                dm = fmax(dm, d);
                 bad |= !isfinite(a) || !isfinite(s) || !isfinite(d) || !isfinite(x) || !(a > 0.0) || !(x > 0.0);
             }
-            for (int o = 1; o <= 2; o <<= 1) gr = fmax(gr, __shfl_xor_sync(0xffffffffu, gr, o));
-            const double skew = n > 0 ? __hiloint2double((int)stat[SYM_STAT_SKEW], 0) : 0.0;
+            for (int o = 1; o <= 2; o <<= 1) {
+                gr = fmax(gr, __shfl_xor_sync(0xffffffffu, gr, o));
+                dm = fmax(dm, __shfl_xor_sync(0xffffffffu, dm, o));
+            }
+            const double off = n > SYM_NB ? __hiloint2double((int)stat[SYM_STAT_OFF], 0) : 0.0;
             const unsigned quad = __ballot_sync(0xffffffffu, bad) >> (lane & ~3) & 15u;
             // one tile is pivoted throughout
-            const int mode = n == 0 ? 0 : quad || !(gr <= 1e6) ? 3 : n <= SYM_NB ? 0 : gr > 1e3 ? 2 : gr > 3.0 || skew > SYM_SKEW_NEWTON ? 1 : 0;
+            const int mode = n == 0 ? 0 : quad || !(gr <= 1e6) ? 3 : n <= SYM_NB ? 0 : gr > 1e3 ? 2 : gr > 3.0 || off * dm > 2e4 ? 1 : 0;
             if (k < m && (tid & 3) == 0) {
                 s_mode[k] = mode;
                 if (n > 0 && blockIdx.x == 0) stat[0] = (unsigned)mode;

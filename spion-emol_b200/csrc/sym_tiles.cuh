@@ -30,9 +30,11 @@ struct SymEntry {
     double* D;              // the inverse of the pivot tile, the pivot tile itself, and sym_skew of the two
     double* out;            // n x n, ld ldo: the inverse, both triangles
     unsigned* stat;         // sym_stat_words(n) words, zero before the sweep: [0] how it was finished, [1 ..] SYM_STEPS Newton
-                            // steps' changes, [4] the largest sym_skew (high word), SYM_STAT_HEAD on sym_stat
+                            // steps' changes, [4] the largest element of A off the
+                            // diagonal tiles (high word), SYM_STAT_HEAD on sym_stat
     int* status;            // DeviceStatus, first failing column; zero before the sweep
     int n, ldo;
+    double skew_max;        // SYM_SKEW_MAX, or infinity: no rows refined
 };
 
 __host__ __device__ inline int sym_tiles_of(int n) { return (n + SYM_NB - 1) / SYM_NB; }
@@ -78,7 +80,7 @@ __device__ __forceinline__ unsigned sym_hi(double v) { return (unsigned)__double
 // tile row, of that row in any Schur complement, of the pivot tile's inverse
 // D_i, and of the inverse's tile row.
 enum SymStat { SYM_OF_A = 0, SYM_OF_SCHUR = 1, SYM_OF_D = 2, SYM_OF_X = 3 };
-constexpr int SYM_STEPS = 3, SYM_STAT_SKEW = 4, SYM_STAT_HEAD = 8;
+constexpr int SYM_STEPS = 3, SYM_STAT_OFF = 4, SYM_STAT_HEAD = 8;
 __host__ __device__ inline size_t sym_stat_words(int n) { return SYM_STAT_HEAD + 4 * (size_t)sym_tiles_of(n); }
 __device__ __forceinline__ unsigned* sym_stat(const SymEntry& e, int i, SymStat q) { return e.stat + SYM_STAT_HEAD + 4 * i + q; }
 // A warp's part of an element block of tile (i, j): it counts for both tile rows.
@@ -384,10 +386,7 @@ __device__ __forceinline__ void sym_diag_store(const SymEntry& e, int K, const S
     s0 = fmax(s0, s1);
 #pragma unroll
     for (int o = 2; o >= 1; o >>= 1) s0 = fmax(s0, __shfl_xor_sync(0xffffffffu, s0, o));
-    if (lane == 0) {
-        sym_skew(e)[C] = s0;
-        atomicMax(e.stat + SYM_STAT_SKEW, sym_hi(s0));
-    }
+    if (lane == 0) sym_skew(e)[C] = s0;
 }
 
 // Packs tile t of entry e from elem(row, column, inside) (the element of a
@@ -426,6 +425,10 @@ __device__ __forceinline__ void sym_pack_tile(const SymEntry& e, int t, SymDiagS
         }
     }
     sym_track(e, m, i, j, SYM_OF_A);
+    if (i != j) {
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) atomicMax(e.stat + SYM_STAT_OFF, m);
+    }
     if (first) {
         __syncthreads();
         sym_diag_invert(sh);
